@@ -11,6 +11,7 @@
 #include <mutex>
 #include <string>
 
+#include "common.cuh"
 #include "fmha_launch.h"
 #include "host_util.h"
 
@@ -141,6 +142,8 @@ __device__ __forceinline__ float load_as(const void* src, int dtype, int64_t i) 
 
 __global__ void fill_kernel(void* dst, int dtype, int64_t n, uint64_t seed, int64_t first, int kind, float scale,
                             float value) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   const uint64_t key = mix64(seed);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float v = value;
@@ -155,6 +158,8 @@ __global__ void fill_kernel(void* dst, int dtype, int64_t n, uint64_t seed, int6
 }
 
 __global__ void convert_kernel(const void* src, int sdt, void* dst, int ddt, int64_t n, float scale) {
+  grid_dependency_launch();
+  grid_dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     store_as(dst, ddt, i, load_as(src, sdt, i) * scale);
 }
@@ -226,8 +231,8 @@ extern "C" int cfk_fill(void* dst, int dtype, int64_t n, uint64_t seed, int64_t 
   const int threads = 256;
   const int64_t want = (n + threads - 1) / threads;
   const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
-  fill_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(dst, dtype, n, seed, first_index, kind, scale, value);
-  return note_cuda(cudaGetLastError(), "fill launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
+  return note_cuda(launch_overlapped(fill_kernel, blocks, threads, 0, (cudaStream_t)stream, dst, dtype, n, seed, first_index,
+                                     kind, scale, value), "fill launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
 }
 
 extern "C" int cfk_convert(const void* src, int src_dtype, void* dst, int dst_dtype, int64_t n, float scale,
@@ -237,8 +242,8 @@ extern "C" int cfk_convert(const void* src, int src_dtype, void* dst, int dst_dt
   const int threads = 256;
   const int64_t want = (n + threads - 1) / threads;
   const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
-  convert_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(src, src_dtype, dst, dst_dtype, n, scale);
-  return note_cuda(cudaGetLastError(), "convert launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
+  return note_cuda(launch_overlapped(convert_kernel, blocks, threads, 0, (cudaStream_t)stream, src, src_dtype, dst, dst_dtype,
+                                     n, scale), "convert launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -115,6 +115,17 @@ __device__ __forceinline__ void settle_if_aborted(volatile uint32_t* cta_abort) 
   }
 }
 
+// ---- programmatic dependent launch -----------------------------------------------------------
+// Launches are made with programmatic stream serialization (host_util.h, launch_overlapped): the CTAs of a launch may
+// become resident while the launch before it in the stream is still running, set up their barriers and tensor memory,
+// and then wait here until that launch has completed and its writes are visible.  Nothing of global memory that a
+// launch before may have written (inputs, status word) is read, and nothing is written, ahead of the wait; every thread
+// executes it, so a launch never completes before its predecessor.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The launch after this one may start filling SMs once every CTA of this launch has executed this (or left): from then
+// on no CTA of this launch is still waiting for an SM.
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // CTA-uniform test of the status word (one thread reads, everybody gets the same answer).
 __device__ __forceinline__ bool cta_should_skip(const int* status) {
   __shared__ int s_skip;

@@ -75,9 +75,10 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const uint32_t bar_o_full = bar_pv_done + 8;
   const uint32_t bar_o_staged = bar_o_full + 8;              // one arrival per softmax warp
   const uint32_t off_misc = (bar_o_staged + 8) - sBar;
-  static_assert(8 * (2 * C::NSLOT + 8) + 8 <= C::BARB, "barrier block overflows");
+  static_assert(8 * (2 * C::NSLOT + 8) + 16 <= C::BARB, "barrier block overflows");
   volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(gBar + off_misc);
   volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(gBar + off_misc + 4);
+  volatile uint32_t* s_skip = reinterpret_cast<volatile uint32_t*>(gBar + off_misc + 8);
   const AbortCtx actx{s_abort, p.status};
 
   const int tid = threadIdx.x;
@@ -107,9 +108,9 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     n_kv = nc < n_kv ? nc : n_kv;
   }
 
-  if (cta_should_skip(p.status)) return;
-
-  if (tid == 0) {
+  // Set-up as in fmha_fwd_sm100.cuh: ahead of the wait for the launch before, with Q and K_0 on their way early.
+  grid_dependency_launch();
+  if (warp == 5 && lane == 0) {
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < C::NSLOT; ++i) {
       mbar_init(bar_kv_full + 8 * i, 1);
@@ -124,21 +125,37 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     mbar_init(bar_o_staged, 4);
     *s_abort = 0u;
     fence_barrier_init();
+    fence_proxy_async_smem();
+    grid_dependency_wait();
+    mbar_arrive_expect_tx(bar_q_full, C::QB);
+    tma_load_5d(sQ, &tm_q, bar_q_full, 0, row0, 0, head, batch);
+    for (int h = 0; h < 2; ++h) {       // the two halves of K_0 are ring indices 0 and 1
+      mbar_arrive_expect_tx(bar_kv_full + 8 * h, C::SLOTB);
+      tma_load_5d(sRing + h * C::SLOTB, &tm_k, bar_kv_full + 8 * h, 0, 0, C::HSPANS * h, head, batch);
+    }
+    tma_prefetch_desc(&tm_v);
+    tma_prefetch_desc(&tm_o);
   }
   if (warp == 4) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(s_tmem_base)), C::TMEM_COLS);
     tmem_relinquish();
   }
-  if (warp == 5 && lane == 0) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
-    tma_prefetch_desc(&tm_o);
-  }
+  if (warp == 5) __syncwarp();
+  grid_dependency_wait();
+  if (tid == 0) *s_skip = (uint32_t)(*reinterpret_cast<const volatile int*>(p.status) != 0);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem_base;
+  if (*s_skip) {                         // a wait of an earlier launch gave up
+    if (warp == 5 && lane == 0) {
+      mbar_wait(bar_q_full, 0, actx, kErrFmhaQFull);
+      for (int h = 0; h < 2; ++h) mbar_wait(bar_kv_full + 8 * h, 0, actx, kErrFmhaKvFull);
+    }
+    __syncthreads();
+    if (warp == 4) tmem_dealloc(tmem_base, C::TMEM_COLS);
+    return;
+  }
 
   // bf16 only: blocks whose first row sees few keys keep P as a two-term sum (hi + lo, lo in columns 64-127 of S_x)
   bool split = false;
@@ -152,9 +169,7 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // =========================== TMA producer ===========================
     // Ring order = order of use: K_0 (two halves), K_1, then for every j: V_j (two halves), K_{j+2}.
     if (lane == 0) {
-      mbar_arrive_expect_tx(bar_q_full, C::QB);
-      tma_load_5d(sQ, &tm_q, bar_q_full, 0, row0, 0, head, batch);
-      int idx = 0;
+      int idx = 2;                           // K_0 was loaded in the set-up
       auto load = [&](const CUtensorMap* tm, int j) -> bool {   // both halves of K_j or V_j
         for (int h = 0; h < 2; ++h, ++idx) {
           const int slot = idx % C::NSLOT;
@@ -165,8 +180,7 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         return true;
       };
-      bool ok = load(&tm_k, 0);
-      if (ok && n_kv > 1) ok = load(&tm_k, 1);
+      bool ok = n_kv > 1 ? load(&tm_k, 1) : true;
       for (int j = 0; j < n_kv && ok; ++j) {
         ok = load(&tm_v, j);
         if (ok && j + 2 < n_kv) ok = load(&tm_k, j + 2);

@@ -57,9 +57,10 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t bar_pv_done = bar_o_staged + 16;            // [2] P in its own buffer: O_t += P_t V_j is complete
   const uint32_t bar_s_read = bar_pv_done + 16;              // [2] shared S buffer: tile t's scores are in registers (4 warps)
   const uint32_t off_misc = (bar_s_read + 16) - sBar;
-  static_assert(8 + 16 * C::NSLOT + 16 + 32 + 16 + 16 + 16 + 16 + 16 <= C::BARB, "barrier block overflows");
+  static_assert(8 + 16 * C::NSLOT + 16 + 32 + 16 + 16 + 16 + 16 + 24 <= C::BARB, "barrier block overflows");
   volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(gBar + off_misc);
   volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(gBar + off_misc + 4);
+  volatile uint32_t* s_skip = reinterpret_cast<volatile uint32_t*>(gBar + off_misc + 8);
   const AbortCtx actx{s_abort, p.status};
 
   const int tid = threadIdx.x;
@@ -99,12 +100,11 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   auto n_of = [&](int t) -> int { return t == 0 ? n_t0 : n_t1; };
   const int n_kv = n_t0 > n_t1 ? n_t0 : n_t1;
 
-  // A launch that finds the status word already set does nothing: once one wait has given up, the
-  // rest of the grid (and later launches) must not each spend their own time limit.
-  if (cta_should_skip(p.status)) return;
-
   // ---- set-up ----
-  if (tid == 0) {
+  // Everything up to grid_dependency_wait() overlaps the launch before this one.  The producer thread sets the barriers
+  // up itself, so that Q and K_0 are on their way before the CTA meets at the __syncthreads.
+  grid_dependency_launch();
+  if (warp == 9 && lane == 0) {
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < C::NSLOT; ++i) {
       mbar_init(bar_kv_full + 8 * i, 1);
@@ -121,21 +121,38 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     *s_abort = 0u;
     fence_barrier_init();
+    fence_proxy_async_smem();
+    grid_dependency_wait();
+    mbar_arrive_expect_tx(bar_q_full, (n_t0 > 0 ? C::TILEB : 0) + (n_t1 > 0 ? C::TILEB : 0));
+    for (int t = 0; t < 2; ++t)
+      if (n_of(t) > 0) tma_load_5d(sQ + t * C::TILEB, &tm_q, bar_q_full, 0, qblk * 256 + t * 128, 0, head, batch);
+    mbar_arrive_expect_tx(bar_kv_full, C::TILEB);
+    tma_load_5d(sRing, &tm_k, bar_kv_full, 0, 0, 0, head, batch);     // K_0 is ring index 0
+    tma_prefetch_desc(&tm_v);
+    tma_prefetch_desc(&tm_o);
   }
   if (warp == 8) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(s_tmem_base)), C::TMEM_COLS);
     tmem_relinquish();
   }
-  if (warp == 9 && lane == 0) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
-    tma_prefetch_desc(&tm_o);
-  }
+  if (warp == 9) __syncwarp();
+  grid_dependency_wait();
+  // A launch that finds the status word already set does nothing: once one wait has given up, the
+  // rest of the grid (and later launches) must not each spend their own time limit.
+  if (tid == 0) *s_skip = (uint32_t)(*reinterpret_cast<const volatile int*>(p.status) != 0);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem_base;
+  if (*s_skip) {
+    if (warp == 9 && lane == 0) {    // the two loads above must have landed before shared memory is given back
+      mbar_wait(bar_q_full, 0, actx, kErrFmhaQFull);
+      mbar_wait(bar_kv_full, 0, actx, kErrFmhaKvFull);
+    }
+    __syncthreads();
+    if (warp == 8) tmem_dealloc(tmem_base, C::TMEM_COLS);
+    return;
+  }
 
   // bf16 only: rows that see few keys get P as a two-term sum (hi + lo), see the P store below.
   bool split = false;
@@ -169,12 +186,8 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
    if (warp == 9) {
     // =========================== TMA producer ===========================
     if (lane == 0 && n_kv > 0) {
-      const uint32_t q_bytes = (n_t0 > 0 ? C::TILEB : 0) + (n_t1 > 0 ? C::TILEB : 0);
-      mbar_arrive_expect_tx(bar_q_full, q_bytes);
-      for (int t = 0; t < 2; ++t)
-        if (n_of(t) > 0) tma_load_5d(sQ + t * C::TILEB, &tm_q, bar_q_full, 0, qblk * 256 + t * 128, 0, head, batch);
-      // Tiles enter the ring in the order the UMMA warp first uses them: K_0, then V_j, K_{j+1}.
-      int idx = 0;
+      // Tiles enter the ring in the order the UMMA warp first uses them: K_0 (loaded in the set-up), then V_j, K_{j+1}.
+      int idx = 1;
       bool ok = true;
       auto load_tile = [&](bool is_v, int j) {
         const int slot = idx % C::NSLOT;
@@ -185,13 +198,11 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tma_load_5d(sRing + slot * C::SLOTB, is_v ? &tm_v : &tm_k, bar_kv_full + 8 * slot, 0, j * C::BN, 0, head, batch);
       };
       if (mode != kSharedS) {
-        load_tile(false, 0);
         for (int j = 0; j < n_kv && ok; ++j) {
           load_tile(true, j);
           if (j + 1 < n_kv && ok) load_tile(false, j + 1);
         }
       } else {   // K_0, K_1, then V_j, K_{j+2}
-        load_tile(false, 0);
         if (n_kv > 1 && ok) load_tile(false, 1);
         for (int j = 0; j < n_kv && ok; ++j) {
           load_tile(true, j);

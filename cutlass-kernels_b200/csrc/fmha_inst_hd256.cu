@@ -20,8 +20,10 @@ static int launch_hd256_e(const FmhaLaunch& L) {
   }
   const dim3 grid((unsigned)((long long)L.p.nqblk * L.p.H * L.p.B), 1, 1);   // 128-row blocks
   for (int it = 0; it < L.iterations; ++it)
-    kern<<<grid, C::NTHREADS, C::SMEM_BYTES, L.stream>>>(L.tm_q, L.tm_k, L.tm_v, L.tm_o, L.p);
-  return note_cuda(cudaGetLastError(), "fmha hd256 launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
+    if (note_cuda(launch_overlapped(kern, grid, C::NTHREADS, C::SMEM_BYTES, L.stream, L.tm_q, L.tm_k, L.tm_v, L.tm_o, L.p),
+                  "fmha hd256 launch") != cudaSuccess)
+      return CFK_ERR_LAUNCH;
+  return CFK_OK;
 }
 
 template <int DT>

@@ -20,10 +20,11 @@ int fmha_launch_e(const FmhaLaunch& L) {
     attr_set_for_device = dev;
   }
   const dim3 grid((unsigned)((long long)L.p.nqblk * L.p.H * L.p.B), 1, 1);
-  for (int it = 0; it < L.iterations; ++it) {
-    kern<<<grid, C::NTHREADS, C::SMEM_BYTES, L.stream>>>(L.tm_q, L.tm_k, L.tm_v, L.tm_o, L.p);
-  }
-  return note_cuda(cudaGetLastError(), "fmha launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
+  for (int it = 0; it < L.iterations; ++it)
+    if (note_cuda(launch_overlapped(kern, grid, C::NTHREADS, C::SMEM_BYTES, L.stream, L.tm_q, L.tm_k, L.tm_v, L.tm_o, L.p),
+                  "fmha launch") != cudaSuccess)
+      return CFK_ERR_LAUNCH;
+  return CFK_OK;
 }
 
 template <int DT, int PT, int HD>

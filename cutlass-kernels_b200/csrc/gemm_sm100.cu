@@ -101,8 +101,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   const int bk = p.tf32 ? C::BK / 2 : C::BK;   // elements per 128-byte stage row
   const int nkb = (p.K + bk - 1) / bk;
 
-  // One decision for the pair: both CTAs skip or both run (pair_should_skip).
-  if (pair_should_skip(p.status)) return;
+  grid_dependency_launch();
   if (tid == 0) {
     for (int i = 0; i < C::NSTAGE; ++i) { mbar_init(bar_full + 8 * i, 2); mbar_init(bar_empty + 8 * i, 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(bar_acc_full + 8 * i, 1); mbar_init(bar_acc_empty + 8 * i, 256); }
@@ -115,11 +114,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
     tmem_relinquish_pair();
   }
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_y); tma_prefetch_desc(&tm_d); }
+  grid_dependency_wait();
   tc_fence_before_sync();
-  __syncthreads();
-  cluster_sync_all();           // the peer's barriers exist before anything is signalled on them
+  // One decision for the pair: both CTAs skip or both run.  Its cluster barrier also says that the peer's barriers
+  // exist before anything is signalled on them.
+  const bool skip = pair_should_skip(p.status);
   tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem_base;
+  if (skip) {
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+    return;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -396,6 +401,8 @@ extern "C" int cfk_gemm(const cfk_gemm_args* a, cfk_stream_t stream) {
   const long long pairs = total < sm_count / 2 ? total : sm_count / 2;   // one CTA pair per two SMs
   const int grid = (int)(2 * pairs);
   for (int it = 0; it < a->iterations; ++it)
-    gemm_kernel<<<grid, GemmCfg::NTHREADS, GemmCfg::SMEM_BYTES, (cudaStream_t)stream>>>(tm_x, tm_y, tm_d, p);
-  return note_cuda(cudaGetLastError(), "gemm launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
+    if (note_cuda(launch_overlapped(gemm_kernel, grid, GemmCfg::NTHREADS, GemmCfg::SMEM_BYTES, (cudaStream_t)stream, tm_x, tm_y,
+                                    tm_d, p), "gemm launch") != cudaSuccess)
+      return CFK_ERR_LAUNCH;
+  return CFK_OK;
 }
