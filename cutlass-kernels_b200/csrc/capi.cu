@@ -1,9 +1,5 @@
 // C-ABI entry points that are not a kernel family of their own: argument validation and dispatch for
-// cfk_fmha_forward, fills / conversions, status handling.  Declarations: include/cfk_b200.h.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-#include <cuda_fp8.h>
-
+// cfk_fmha_forward, fills, status handling.  Declarations: include/cfk_b200.h.
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -12,6 +8,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "element_io.cuh"
 #include "fmha_launch.h"
 #include "host_util.h"
 
@@ -113,7 +110,7 @@ int encode_bshd(CUtensorMap* map, int dtype, const void* base, int batch, int se
 }
 
 // ------------------------------------------------------------------------------------------------
-// fills and conversions
+// fills
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   z += 0x9e3779b97f4a7c15ull;
@@ -122,23 +119,6 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   return z ^ (z >> 31);
 }
 __device__ __forceinline__ float unit_open(uint32_t x) { return ((float)(x >> 8) + 0.5f) * (1.0f / 16777216.0f); }
-
-__device__ __forceinline__ void store_as(void* dst, int dtype, int64_t i, float v) {
-  if (dtype == CFK_FP16) reinterpret_cast<__half*>(dst)[i] = __float2half_rn(v);
-  else if (dtype == CFK_BF16) reinterpret_cast<__nv_bfloat16*>(dst)[i] = __float2bfloat16_rn(v);
-  else if (dtype == CFK_E4M3)
-    reinterpret_cast<uint8_t*>(dst)[i] = (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
-  else reinterpret_cast<float*>(dst)[i] = v;
-}
-__device__ __forceinline__ float load_as(const void* src, int dtype, int64_t i) {
-  if (dtype == CFK_FP16) return __half2float(reinterpret_cast<const __half*>(src)[i]);
-  if (dtype == CFK_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(src)[i]);
-  if (dtype == CFK_E4M3) {
-    __half_raw h = __nv_cvt_fp8_to_halfraw(reinterpret_cast<const uint8_t*>(src)[i], __NV_E4M3);
-    return __half2float(__half(h));
-  }
-  return reinterpret_cast<const float*>(src)[i];
-}
 
 __global__ void fill_kernel(void* dst, int dtype, int64_t n, uint64_t seed, int64_t first, int kind, float scale,
                             float value) {
@@ -155,13 +135,6 @@ __global__ void fill_kernel(void* dst, int dtype, int64_t n, uint64_t seed, int6
     }
     store_as(dst, dtype, i, kind == 3 ? v : v * scale);
   }
-}
-
-__global__ void convert_kernel(const void* src, int sdt, void* dst, int ddt, int64_t n, float scale) {
-  grid_dependency_launch();
-  grid_dependency_wait();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    store_as(dst, ddt, i, load_as(src, sdt, i) * scale);
 }
 
 // Tunables (process-wide).  Defaults are the measured best on B200.
@@ -233,17 +206,6 @@ extern "C" int cfk_fill(void* dst, int dtype, int64_t n, uint64_t seed, int64_t 
   const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
   return note_cuda(launch_overlapped(fill_kernel, blocks, threads, 0, (cudaStream_t)stream, dst, dtype, n, seed, first_index,
                                      kind, scale, value), "fill launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
-}
-
-extern "C" int cfk_convert(const void* src, int src_dtype, void* dst, int dst_dtype, int64_t n, float scale,
-                           cfk_stream_t stream) {
-  if (!src || !dst || n < 0 || !valid_dtype(src_dtype) || !valid_dtype(dst_dtype)) return CFK_ERR_INVALID_ARG;
-  if (n == 0) return CFK_OK;
-  const int threads = 256;
-  const int64_t want = (n + threads - 1) / threads;
-  const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
-  return note_cuda(launch_overlapped(convert_kernel, blocks, threads, 0, (cudaStream_t)stream, src, src_dtype, dst, dst_dtype,
-                                     n, scale), "convert launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
 }
 
 // ------------------------------------------------------------------------------------------------
