@@ -224,6 +224,30 @@ static bool resolve_strides(const int64_t in[3], int64_t out[3], int S, int H, i
   return true;
 }
 
+// Few query rows against a long cache (fmha_decode_sm100.cuh).  It re-reads K and V per 16 query rows and its arithmetic is
+// the warps' own, so it wins where the 256-row kernel has rows or SMs to spare.  us, bf16, 256-row kernel / this one:
+//   up to 32 rows: d = 128, 200 heads, 8 x 1508: 43.1 / 30.1, 32 x 1532: 43.5 / 35.5; d = 64, 64 heads, 32 x 6032: 56.8 / 24.6;
+//   up to 128 rows, while every group of 16 rows can have an SM: d = 128, 24 heads, 64 x 6064: 70.0 / 30.9, 8 heads,
+//   128 x 1628: 22.0 / 11.4; beyond that it loses: 64 heads, 64 x 1564: 24.1 / 23.5, 200 heads, 64 x 364: 22.4 / 27.3; short
+//   caches of so many rows are launch-bound either way;
+//   d = 256, where the other kernel already has one 128-row tile per CTA and a tile here fills an SM: four CTAs or more per
+//   group, 24 heads, 8 x 6008: 62.6 / 29.6; with fewer it is even: 64 heads, 16 x 1516: 23.4 / 25.2.
+static bool decode_is_faster(long long groups, int sq, int skv, int head_dim) {
+  constexpr int kSMs = 148;
+  if (groups > 0x7fffffffLL / 8) return false;
+  if (head_dim == 256) return sq <= 128 && skv >= 1024 && 4 * groups <= kSMs;
+  return sq <= 32 || (sq <= 128 && skv >= 1024 && groups <= kSMs);
+}
+
+// CTAs (a cluster) per group of 16 rows: as many as are resident at once, with two tiles of keys each at least; 8 is the
+// portable limit.  us for 1 / 2 / 4 / 8, bf16 d = 128: 128 heads x 6001 keys 64.2 / 62.9 / 73.9 / 70.5; 32 heads x 4096
+// 30.9 / 19.9 / 16.3 / 16.0; 256 heads x 1024 24.6 / 32.5 / 33.3 / 46.1; 2 heads x 65536 410 / 210 / 108 / 57.5.
+static int decode_splits(long long groups, int ntiles, int resident) {
+  int s = 1;
+  while (s < 8 && groups * 2 * s <= resident && ntiles >= 4 * s) s *= 2;
+  return s;
+}
+
 // Argument checks, TMA descriptors, kernel parameters and kernel choice of one FMHA call: everything of the launch
 // except the status pointer and the stream, which the two entry points supply (allocated block / static array).
 // *p_dtype receives the type P is rounded to (and V is stored in).
@@ -259,20 +283,31 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   FmhaLaunch& L = *out;
   std::memset(&L, 0, sizeof(L));
   int rc;
-  if ((rc = encode_bshd(&L.tm_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], 128)))
-    return rc;
-  // head dimension 256: K and V tiles travel as two halves of 128 columns (two 128-byte spans) each
-  const int kv_spans = a->head_dim == 256 ? esz : 0;   // 128 columns = esz spans of 128 bytes
-  if ((rc = encode_bshd(&L.tm_k, a->dtype, a->k, a->batch, a->seqlen_kv, a->heads, a->head_dim, ks[0], ks[1], ks[2], 128, kv_spans)))
-    return rc;
-  if ((rc = encode_bshd(&L.tm_v, vdt, a->v, a->batch, a->seqlen_kv, a->heads, a->head_dim, vs[0], vs[1], vs[2], 128, kv_spans)))
-    return rc;
-  if ((rc = encode_bshd(&L.tm_o, a->out_dtype, a->o, a->batch, a->seqlen_q, a->heads, a->head_dim, os[0], os[1], os[2], 128)))
-    return rc;
-
   L.variant = g_tunable[CFK_TUNE_FMHA_KERNEL].load();
   if (L.variant == 1 && (a->dtype == CFK_E4M3 || a->head_dim != 128)) L.variant = 0;
   if (a->head_dim == 256) L.variant = 0;
+  const long long groups16 = (long long)a->batch * a->heads * ((a->seqlen_q + 15) / 16);
+  const bool decode = L.variant == 0 && !a->s_dump && decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim);
+  if (decode) L.variant = 3;
+  const int q_rows = decode ? 16 : 128, kv_rows = decode ? decode_tile_keys(a->head_dim, dtype_size(vdt)) : 128;
+  if ((rc = encode_bshd(&L.tm_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], q_rows)))
+    return rc;
+  // head dimension 256: K and V tiles travel as two halves of 128 columns (two 128-byte spans) each
+  const int kv_spans = a->head_dim == 256 && !decode ? esz : 0;   // 128 columns = esz spans of 128 bytes
+  if ((rc = encode_bshd(&L.tm_k, a->dtype, a->k, a->batch, a->seqlen_kv, a->heads, a->head_dim, ks[0], ks[1], ks[2], kv_rows, kv_spans)))
+    return rc;
+  if ((rc = encode_bshd(&L.tm_v, vdt, a->v, a->batch, a->seqlen_kv, a->heads, a->head_dim, vs[0], vs[1], vs[2], kv_rows, kv_spans)))
+    return rc;
+  if ((rc = encode_bshd(&L.tm_o, a->out_dtype, a->o, a->batch, a->seqlen_q, a->heads, a->head_dim, os[0], os[1], os[2], 128)))
+    return rc;
+  if (decode) {
+    L.dec.o = a->o;
+    L.dec.o_b = os[0]; L.dec.o_s = os[1]; L.dec.o_h = os[2];
+    L.dec.nqb = (a->seqlen_q + 15) / 16;
+    L.dec.splits = decode_splits(groups16, (a->seqlen_kv + kv_rows - 1) / kv_rows,
+                                 148 * decode_ctas_per_sm(a->head_dim, esz, dtype_size(vdt)));
+  }
+
   L.grid_ctas = g_tunable[CFK_TUNE_FMHA_GRID].load();
   if (L.variant == 1) {   // CTA-pair kernel: each CTA loads 64 keys of a K tile and one 64-column span of a V tile
     if ((rc = encode_bshd(&L.tm_k_half, a->dtype, a->k, a->batch, a->seqlen_kv, a->heads, a->head_dim, ks[0], ks[1], ks[2], 64)))

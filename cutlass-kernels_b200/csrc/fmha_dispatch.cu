@@ -6,6 +6,11 @@
 namespace cfk {
 
 int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L) {
+  if (L.variant == 3) {
+    if (dtype == CFK_FP16) return fmha_launch_decode_f16(L, head_dim);
+    if (dtype == CFK_BF16) return fmha_launch_decode_bf16(L, head_dim);
+    return p_dtype == CFK_FP16 ? fmha_launch_decode_e4m3_f16(L, head_dim) : fmha_launch_decode_e4m3(L, head_dim);
+  }
   if (head_dim == 256) {
     if (dtype == CFK_FP16 && p_dtype == CFK_FP16) return fmha_launch_hd256_f16(L);
     if (dtype == CFK_BF16 && p_dtype == CFK_BF16) return fmha_launch_hd256_bf16(L);

@@ -13,9 +13,11 @@ namespace cfk {
 struct FmhaLaunch {
   CUtensorMap tm_q, tm_k, tm_v, tm_o;
   CUtensorMap tm_k_half, tm_v_half;   // CTA-pair kernel: boxes of 64 keys x all columns / 128 keys x one 64-column span
-  int variant;                        // 0 one CTA per 256 query rows, 1 CTA pairs, 2 persistent, one tile per CTA (see cfk_b200.h)
+  int variant;                        // 0 one CTA per 256 query rows, 1 CTA pairs, 2 persistent, one tile per CTA (see cfk_b200.h),
+                                      // 3 a few query rows against a long cache (fmha_decode_sm100.cuh); never set by the caller
   int grid_ctas;                      // variant 2: CTAs of the persistent grid (0 = one per SM)
   FmhaParams p;
+  FmhaDecodeParams dec;               // variant 3: the part of it that is not `p`
   int iterations;
   int exp_emu;   // 0..3: share (in quarters) of the exponentials computed on the FMA pipe
   cudaStream_t stream;
@@ -44,6 +46,12 @@ int fmha_launch_persist_e4m3_e4m3_64(const FmhaLaunch&);
 int fmha_launch_persist_e4m3_e4m3_128(const FmhaLaunch&);
 int fmha_launch_pair_f16(const FmhaLaunch&);
 int fmha_launch_pair_bf16(const FmhaLaunch&);
+
+// variant 3: tm_q boxes are 16 rows, tm_k / tm_v boxes decode_tile_keys() keys x all columns
+int fmha_launch_decode_f16(const FmhaLaunch&, int head_dim);
+int fmha_launch_decode_bf16(const FmhaLaunch&, int head_dim);
+int fmha_launch_decode_e4m3(const FmhaLaunch&, int head_dim);
+int fmha_launch_decode_e4m3_f16(const FmhaLaunch&, int head_dim);
 
 int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L);
 

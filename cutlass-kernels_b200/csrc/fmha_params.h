@@ -1,5 +1,6 @@
 // Kernel parameter block and status codes of the FMHA kernel family (host and device).
 #pragma once
+#include <stdint.h>
 
 namespace cfk {
 
@@ -9,7 +10,8 @@ constexpr int kDtF16 = 0, kDtBF16 = 1, kDtE4M3 = 2;
 constexpr int kErrFmhaQFull = 101, kErrFmhaKvFull = 102, kErrFmhaKvEmpty = 103, kErrFmhaSFull = 104,
               kErrFmhaPFull = 105, kErrFmhaOFull = 106, kErrFmhaOStaged = 107, kErrFmhaSFree = 108,
               kErrFmhaPvDone = 109, kErrFmhaMaxPub = 110, kErrFmhaPvDone256 = 111, kErrFmhaRowMax = 112,
-              kErrFmhaSRead = 113, kErrFmhaOFree = 115, kErrFmhaStats = 117, kErrFmhaCorrPv = 118;
+              kErrFmhaSRead = 113, kErrFmhaOFree = 115, kErrFmhaStats = 117, kErrFmhaCorrPv = 118,
+              kErrDecodeFull = 121, kErrDecodeEmpty = 122;
 
 struct FmhaParams {
   int B, H, Sq, Skv;
@@ -27,6 +29,21 @@ struct FmhaParams {
   void* s_dump;      // optional debug output [B][H][Sq][Skv]: raw Q K^T (16-bit); see cfk_b200.h
   int s_dump_bf16;   // element type of s_dump: 0 fp16, 1 bf16
   int* status;       // device status word
+};
+
+// The kernel for a few query rows (fmha_decode_sm100.cuh)
+constexpr int decode_tile_keys(int head_dim, int v_bytes) { return head_dim * v_bytes >= 256 ? 64 : 128; }
+// CTAs that share an SM: by shared memory (a tile of K and V of 64 KB), by registers (the output takes head_dim / 2)
+constexpr int decode_ctas_per_sm(int head_dim, int k_bytes, int v_bytes) {
+  return decode_tile_keys(head_dim, v_bytes) * head_dim * (k_bytes + v_bytes) >= 65536 ? 1 : (head_dim == 256 ? 2 : 3);
+}
+struct FmhaDecodeParams {
+  FmhaParams p;
+  void* o;
+  int64_t o_b, o_s, o_h;   // element strides of O
+  int nqb;                 // groups of 16 query rows
+  int nslot;               // slots of the ring of K and V tiles
+  int splits;              // CTAs (a cluster) that share the keys of one (batch, head, group of rows)
 };
 
 }  // namespace cfk

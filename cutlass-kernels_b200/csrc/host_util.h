@@ -19,20 +19,29 @@ cudaError_t note_cuda(cudaError_t e, const char* what);
 // Plain back-to-back launches of a kernel of a few microseconds repeat every 4.1, 6.2 or 8.2 us on B200 (steps of 2.05 us
 // whatever the kernel does); launched this way the period is the kernel's own work plus about 1.2 us, and the host side
 // of a launch takes 2.1 us instead of 2.6.
+// `cluster` > 1: in clusters of so many CTAs along x (for kernels without a cluster size of their own).
 template <class... KArgs, class... Args>
-inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                     const Args&... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t launch_overlapped_in(int cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                        cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                     const Args&... args) {
+  return launch_overlapped_in(1, kern, grid, block, smem, stream, args...);
 }
 
 // Device pointer to the 256-byte status block of the current device (int[64]; word 0 is the status

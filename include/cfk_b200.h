@@ -55,9 +55,10 @@ typedef struct cfk_fmha_args {
   int dtype;      /* cfk_dtype of Q, K and V: FP16, BF16 or E4M3 */
   int out_dtype;  /* cfk_dtype of O: FP16 or BF16 */
   int p_split_keys; /* P (unnormalised probabilities) is rounded to the input type before P*V, as the
-                       reference does (fmha_consumer.h:54).  bf16 only: 256-row query blocks whose first
-                       row sees fewer keys than this keep P as a two-term bf16 sum (hi + lo, two MMAs),
-                       because with few keys bf16's 8-bit rounding of P is not averaged out.
+                       reference does (fmha_consumer.h:54).  bf16 only: query blocks (256 rows; 128 at head
+                       dimension 256; 16 where few rows meet a long cache) whose first row sees fewer keys than
+                       this keep P as a two-term bf16 sum (hi + lo, two MMAs), because
+                       with few keys bf16's 8-bit rounding of P is not averaged out.
                        -1 = default (1024), 0 = never.  Ignored for fp16 / e4m3. */
   int batch, heads, seqlen_q, seqlen_kv, head_dim;
   const void* q;
@@ -169,7 +170,10 @@ const char* cfk_last_cuda_error(void);
  *                           by input type and head dimension, the measured best.
  *   CFK_TUNE_FMHA_GROUP_MB  causal only: heads are scheduled in groups whose K and V total at most
  *                           this many MiB (so they share L2), heaviest query blocks first.
- *   CFK_TUNE_FMHA_KERNEL    which FMHA kernel runs: 0 one CTA per 256 query rows (two 128-row tiles side by side);
+ *   CFK_TUNE_FMHA_KERNEL    which FMHA kernel runs: 0 one CTA per 256 query rows (two 128-row tiles side by side), except that
+ *                           few query rows (up to 32, or up to 128 with few heads and a long cache) run in a kernel
+ *                           that splits the keys over a cluster, so that how a call is cut into heads can change the
+ *                           last bit there;
  *                           1 pairs of CTAs (two SMs per 256 rows, tcgen05 cta_group::2; 16-bit inputs with head
  *                           dimension 128 only, other shapes run kernel 0); 2 a persistent grid whose CTAs take one
  *                           128-row tile at a time, with the scores double-buffered, both softmax warpgroups on the

@@ -1,0 +1,62 @@
+"""Few query rows against a long cache run in a kernel that splits the keys over the CTAs of a cluster.  Sizes are the
+edges of its tiles (16 rows, 64 or 128 keys, a quarter of that per warp), of the split (one tile more or less than a CTA's
+share, CTAs without a visible key) and of the rule that sends a call to it.  Tolerances are those of test_fmha_gpu.py."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import make_qkv, run_fmha
+from test_fmha_gpu import check
+
+pytestmark = pytest.mark.gpu
+
+# (B, H, Sq, Skv): 1 to 8 CTAs per group of rows, whole and ragged tiles
+SHAPES = [(1, 1, 1, 1), (2, 3, 1, 63), (1, 2, 3, 64), (1, 2, 16, 65), (2, 1, 17, 128), (1, 3, 9, 129), (1, 2, 32, 33),
+          (3, 5, 1, 777), (1, 1, 7, 4099), (160, 1, 2, 300), (1, 1, 33, 1024), (1, 2, 100, 1500), (75, 2, 16, 200)]
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("dtype", [0, 1, 2])
+@pytest.mark.parametrize("causal", [False, True])
+def test_few_rows_match_the_oracle(lib, cuda, oracle, D, dtype, causal):
+    for i, (B, H, Sq, Skv) in enumerate(SHAPES):
+        low, f32, scales = make_qkv(dtype, B, Sq, Skv, H, D, seed=500 + i)
+        got, stats = run_fmha(lib, low, scales, dtype, causal)
+        check(oracle, got, stats, f32, 1.0 / math.sqrt(D), causal, dtype)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_few_rows_hybrid_and_a_head_range_of_a_wider_tensor(lib, cuda, oracle, D):
+    """e4m3 Q and K with fp16 V (the hybrid mode), heads 1 and 2 of five: strides of the whole tensor, and the other heads
+    of O and everything behind the last row stay as they were."""
+    B, H, HT, Sq, Skv = 2, 2, 5, 5, 700
+    (q, k, _), (qf, kf, _), (qs, ks, _) = make_qkv(2, B, Sq, Skv, HT, D, seed=77)
+    v = torch.randn(B, Skv, HT, D, generator=torch.Generator().manual_seed(78)).half()
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    o = torch.full((B, Sq, HT, D), -7.0, dtype=torch.float16, device="cuda")
+    lse = torch.zeros(B, H, Sq, device="cuda")
+    at = [t.data_ptr() + D * t.element_size() for t in (qd, kd, vd, o)]
+    sq, skv = (Sq * HT * D, HT * D, D), (Skv * HT * D, HT * D, D)
+    lib.fmha_forward(*at, dtype=2, batch=B, heads=H, seqlen_q=Sq, seqlen_kv=Skv, head_dim=D, softmax_scale=D ** -0.5,
+                     causal=True, lse=lse, q_descale=qs, k_descale=ks, v_fp16=True, q_stride=sq, k_stride=skv,
+                     v_stride=skv, o_stride=sq)
+    lib.check_device()
+    cut = lambda x: np.ascontiguousarray(x[:, :, 1:3])    # noqa: E731
+    check(oracle, cut(o.float().cpu().numpy()), {}, (cut(qf), cut(kf), cut(v.float().numpy())), D ** -0.5, True, 0)
+    rest = o.clone()
+    rest[:, :, 1:3] = -7.0
+    assert bool((rest == -7.0).all())
+
+
+def test_few_rows_keep_infinite_scores_and_large_steps_of_the_maximum(lib, cuda, oracle):
+    """The running maximum moves by far more than the 2^8 it may lag, late and in one warp's keys only; a key whose scores
+    are so low that its probability is zero changes nothing."""
+    low, _, scales = make_qkv(0, 1, 2, 900, 1, 128, seed=9)
+    q, k, v = low
+    k[0, 850] = q[0, 0, 0:1] * 3
+    k[0, 10] = -q[0, 0, 0:1] * 50
+    f32 = [x.float().numpy() for x in (q, k, v)]
+    got, stats = run_fmha(lib, (q, k, v), scales, 0, False)
+    check(oracle, got, stats, f32, 1.0 / math.sqrt(128), False, 0)
