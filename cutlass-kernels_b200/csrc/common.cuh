@@ -348,6 +348,14 @@ __device__ __forceinline__ void umma_commit_e(uint32_t bar, uint32_t leader) {
                  ::"r"(bar), "r"(leader) : "memory");
 }
 
+// cta_group::2: the barrier at this shared-memory offset in every CTA of `cta_mask` (ranks within the cluster) receives the
+// arrival: one commit (about 100 clk of the issuing warp) frees a stage in both CTAs of a pair.
+__device__ __forceinline__ void umma_commit_pair_e(uint32_t bar, uint16_t cta_mask, uint32_t leader) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+               ::"r"(bar), "h"(cta_mask), "r"(leader) : "memory");
+}
+
 // The mbarrier receives one arrival once every tcgen05 operation issued so far by this thread is done.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -371,21 +379,34 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The skip decision of a CTA pair (see cta_should_skip), taken ONCE for the pair: if each CTA read the status word
-// for itself, another CTA's wait could give up between the two reads, one CTA of the pair would return and its peer
+// The skip decision of a cluster (see cta_should_skip), taken ONCE for all its CTAs: if each CTA read the status word
+// for itself, another CTA's wait could give up between two reads, one CTA of a pair would return and its peer
 // would go on to allocate tensor memory for the pair (which has no time limit) and to signal barriers in the shared
-// memory of a CTA that is gone.  Rank 0 reads the word and stores the decision into both CTAs' shared memory; after
-// the cluster barrier both branch on their own copy.  Every thread of both CTAs must call this.
-__device__ __forceinline__ bool pair_should_skip(const int* status) {
-  __shared__ uint32_t s_pair_skip;
+// memory of a CTA that is gone.  Rank 0 reads the word and stores the decision into every CTA's shared memory; after
+// the cluster barrier each branches on its own copy.  Every thread of every CTA must call this.
+__device__ __forceinline__ bool cluster_should_skip(const int* status, int ctas) {
+  __shared__ uint32_t s_cluster_skip;
   if (threadIdx.x == 0 && cluster_ctarank() == 0) {
     const uint32_t v = (uint32_t)(*reinterpret_cast<const volatile int*>(status) != 0);
-    const uint32_t here = smem_u32(&s_pair_skip);
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(here, 0)), "r"(v) : "memory");
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(here, 1)), "r"(v) : "memory");
+    const uint32_t here = smem_u32(&s_cluster_skip);
+    for (int c = 0; c < ctas; ++c)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(here, (uint32_t)c)), "r"(v) : "memory");
   }
-  cluster_sync_all();   // release / acquire at cluster scope: the peer's copy is written before anyone reads
-  return *reinterpret_cast<volatile uint32_t*>(&s_pair_skip) != 0u;
+  cluster_sync_all();   // release / acquire at cluster scope: the copies are written before anyone reads
+  return *reinterpret_cast<volatile uint32_t*>(&s_cluster_skip) != 0u;
+}
+__device__ __forceinline__ bool pair_should_skip(const int* status) { return cluster_should_skip(status, 2); }
+// Reads of another CTA's shared memory (addresses from map_to_cta)
+__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_shared_cluster_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr) : "memory");
+  return v;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");

@@ -92,18 +92,6 @@ __device__ __forceinline__ uint32_t tile_piece(int row, int even, int bit) {
   const int x = SPANB == 128 ? (row & 7) : ((row >> 1) & 3);
   return (uint32_t)((even / CPS) * (ROWS * SPANB) + row * SPANB + (((even % CPS) << 4) ^ ((bit ^ x) << 4)));
 }
-__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ld_shared_cluster_f32x4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr) : "memory");
-  return v;
-}
-
 template <int DT, int PT, int HD>
 __global__ void __launch_bounds__(160, (DecodeCfg<DT, PT, HD>::CTAS))
 fmha_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,

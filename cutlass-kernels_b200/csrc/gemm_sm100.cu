@@ -3,13 +3,13 @@
 // It stands where the reference has gemm<> / gemm_device (src/cute-gemm-tma-gma/gemm.cu:336-463,
 // 57-334): that kernel is a single-stage TMA -> WGMMA loop that stores register accumulators straight
 // to global memory, ignores alpha / beta and accumulates in the output type.  Here a pair of CTAs on two
-// SMs (a cluster of 2, tcgen05 cta_group::2) computes a 256 x 256 tile:
+// SMs (tcgen05 cta_group::2) computes a tile of 256 rows x TN columns, TN = 256, 128 or 64:
 //
-//   warp 0     TMA producer: this CTA's 128 rows of X and its 128 rows of Y per 64-wide k-block, into a
-//              6-stage ring; both CTAs signal the same barrier in the leader (no multicast: each CTA
+//   warp 0     TMA producer: this CTA's 128 rows of X and its TN / 2 rows of Y per 64-wide k-block, into a
+//              ring of 6 or 4 stages; both CTAs signal the same barrier in the leader (no multicast: each CTA
 //              fetches only what its own SM consumes)
-//   warp 1     UMMA issuer (leader CTA only): 256 x 256 x 16 tcgen05.mma over the pair, two accumulator
-//              buffers of 256 TMEM columns per CTA
+//   warp 1     UMMA issuer (leader CTA only): 256 x TN x 16 tcgen05.mma over the pair, two accumulator
+//              buffers of TN TMEM columns per CTA
 //   warps 2-5  epilogue: TMEM -> registers -> alpha/beta -> output type -> a swizzled staging tile in shared
 //              memory (128 rows x 128 bytes, two of them) -> TMA store, overlapped with the next tile's main
 //              loop.  (The reference writes its register accumulators to global memory thread by thread,
@@ -20,10 +20,16 @@
 // 8 row-tiles so that concurrently running tiles share X and Y panels in L2.  The reference's column-major
 // C (gemm.cu:388-389) is the row-major D of the swapped problem (X = B, Y = A), so one kernel serves both
 // output orders.
+//
+// Where the tiles of D are too few for the SMs, `splits` pairs share one tile: a cluster of 2 * splits CTAs, each pair with a
+// part of the reduction.  At the end every CTA leaves its fp32 accumulator, except the columns it is going to finish itself,
+// in its shared memory (the ring is free by then); after a cluster barrier it adds the other pairs' parts of its columns
+// through distributed shared memory, in pair order, and writes them.  No workspace, and the result does not depend on timing.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <cstring>
+#include <utility>
 
 #include "common.cuh"
 #include "host_util.h"
@@ -42,39 +48,97 @@ struct GemmParams {
   float alpha, beta;
   int bf16;
   int tf32;              // operands and D are fp32; the tensor core runs them as tf32 (kind::tf32, 8 elements per k-step)
-  int tiles_r, tiles_c;  // 256 x 256 tiles
+  int tiles_r, tiles_c;  // tiles of 256 x TN
+  int splits;            // pairs that share a tile, each with a part of the reduction
+  int direct;            // one cluster per tile, which writes D from registers (with a split, or with `trans`)
+  int trans;             // X holds the columns of D and Y its rows: D[c][r], still with leading dimension ldd
   int* status;
 };
 
+template <int TN_>
 struct GemmCfg {
-  static constexpr int BM = 128, BNH = 128, BK = 64;         // per CTA: rows of X, rows of Y, k extent
-  static constexpr int TILE = 256;                            // tile edge of the CTA pair
-  static constexpr int XB = BM * BK * 2, YB = BNH * BK * 2;   // bytes per stage
-  static constexpr int NSTAGE = 6;
+  static constexpr int TM = 256, TN = TN_;                    // tile of the CTA pair
+  static constexpr int BM = 128, BNH = TN / 2, BK = 64;       // per CTA: rows of X, rows of Y, k extent
+  // k-blocks per stage: a round of the producer and of the UMMA warp (barrier wait, announced bytes, commit) takes about 400
+  // clk, which a 256-wide tile hides behind 512 clk of MMA per k-block and a narrower one does not.
+  static constexpr int KSUB = TN == 256 ? 1 : 2;
+  static constexpr int XSUB = BM * BK * 2, YSUB = BNH * BK * 2;           // bytes per k-block
+  static constexpr int XB = KSUB * XSUB, YB = KSUB * YSUB;                // bytes per stage
+  static constexpr int NSTAGE = TN == 256 ? 6 : 4;
   static constexpr int STAGEB = 128 * 128;                    // output staging tile: 128 rows x 128 bytes
   static constexpr int SMEM_BYTES = 1024 + NSTAGE * (XB + YB) + 2 * STAGEB + 256;
   static constexpr int NTHREADS = 192;
-  static constexpr int BAND = 8;
+  static constexpr int UNITS = TN / 32, UNITB = 128 * 32 * 4; // split: 32 columns of a CTA's accumulator in shared memory
+  static_assert(UNITS * UNITB <= NSTAGE * (XB + YB), "split: the accumulator is handed over in the ring");
+  static_assert(8 * (2 * NSTAGE + 8) + 8 <= 256, "barrier block overflows");
 };
+constexpr int kGemmBand = 8;
 
 __device__ __forceinline__ void tile_coords(int tile, int tiles_r, int tiles_c, int& tr, int& tc, int& batch) {
   const int per_batch = tiles_r * tiles_c;
   batch = tile / per_batch;
   int t = tile - batch * per_batch;
-  const int band_tiles = GemmCfg::BAND * tiles_c;
+  const int band_tiles = kGemmBand * tiles_c;
   const int band = t / band_tiles;
-  const int first_r = band * GemmCfg::BAND;
-  const int rows_in_band = (tiles_r - first_r) < GemmCfg::BAND ? (tiles_r - first_r) : GemmCfg::BAND;
+  const int first_r = band * kGemmBand;
+  const int rows_in_band = (tiles_r - first_r) < kGemmBand ? (tiles_r - first_r) : kGemmBand;
   t -= band * band_tiles;
   tr = first_r + t % rows_in_band;
   tc = t / rows_in_band;
   if (band & 1) tc = tiles_c - 1 - tc;   // back and forth: a band starts on the Y panels the band before it ended on
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+// The beta term.  32 columns of a row of the source matrix, from element `at` on, `cols` of which exist, are read ahead of
+// their use: a read takes about a microsecond, and the epilogue would otherwise wait for one per 32 columns.
+struct SourceRow { uint4 x[8]; };     // 8 pieces of 4 fp32, or 4 of 8 16-bit values
+__device__ __forceinline__ void load_source(SourceRow& s, const GemmParams& p, size_t at, int cols) {
+  if (p.tf32) {
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.src) + at);
+#pragma unroll
+    for (int g = 0; g < 8; ++g) s.x[g] = g * 4 < cols ? src[g] : make_uint4(0u, 0u, 0u, 0u);
+  } else {
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.src) + at);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) s.x[g] = g * 8 < cols ? src[g] : make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+__device__ __forceinline__ void add_source(float (&v)[32], const GemmParams& p, const SourceRow& s) {
+  if (p.tf32) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      v[g * 4] += p.beta * __uint_as_float(s.x[g].x); v[g * 4 + 1] += p.beta * __uint_as_float(s.x[g].y);
+      v[g * 4 + 2] += p.beta * __uint_as_float(s.x[g].z); v[g * 4 + 3] += p.beta * __uint_as_float(s.x[g].w);
+    }
+  } else {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint32_t ow[4] = {s.x[g].x, s.x[g].y, s.x[g].z, s.x[g].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float lo, hi;
+        if (p.bf16) {
+          lo = __uint_as_float(ow[i] << 16);
+          hi = __uint_as_float(ow[i] & 0xffff0000u);
+        } else {
+          const __half2 hh = *reinterpret_cast<const __half2*>(&ow[i]);
+          lo = __low2float(hh);
+          hi = __high2float(hh);
+        }
+        v[g * 8 + 2 * i] += p.beta * lo;
+        v[g * 8 + 2 * i + 1] += p.beta * hi;
+      }
+    }
+  }
+}
+__device__ __forceinline__ uint32_t pack_out(bool bf16, float lo, float hi) {
+  return bf16 ? pack_bf16x2(lo, hi) : pack_f16x2(lo, hi);
+}
+
+template <int TN>
+__global__ void __launch_bounds__(192, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y,
             const __grid_constant__ CUtensorMap tm_d, const GemmParams p) {
-  using C = GemmCfg;
+  using C = GemmCfg<TN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -95,11 +159,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   const AbortCtx actx{s_abort, p.status};
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t rank = cluster_ctarank();
-  const int pair_id = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const uint32_t crank = cluster_ctarank(), rank = crank & 1u;   // rank within the pair; even = the pair's leader
+  const int part = (int)(crank >> 1);                            // which part of the reduction (0 without a split)
+  const int pair_id = (int)(blockIdx.x >> 1) / p.splits, n_pairs = (int)(gridDim.x >> 1) / p.splits;   // tiles in flight
   const int total_tiles = p.tiles_r * p.tiles_c * p.L;
-  const int bk = p.tf32 ? C::BK / 2 : C::BK;   // elements per 128-byte stage row
-  const int nkb = (p.K + bk - 1) / bk;
+  const int bk = p.tf32 ? C::BK / 2 : C::BK;   // elements per 128-byte row of a k-block
+  const int nks_all = (p.K + bk * C::KSUB - 1) / (bk * C::KSUB);
+  const int ks0 = nks_all * part / p.splits, nks = nks_all * (part + 1) / p.splits - ks0;   // this pair's stages of k-blocks
 
   grid_dependency_launch();
   if (tid == 0) {
@@ -110,19 +176,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(s_tmem_base)), 512);
+    tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(s_tmem_base)), 2 * TN);
     tmem_relinquish_pair();
   }
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_y); tma_prefetch_desc(&tm_d); }
   grid_dependency_wait();
   tc_fence_before_sync();
-  // One decision for the pair: both CTAs skip or both run.  Its cluster barrier also says that the peer's barriers
+  // One decision for the cluster: all CTAs skip or all run.  Its cluster barrier also says that the peer's barriers
   // exist before anything is signalled on them.
-  const bool skip = pair_should_skip(p.status);
+  const bool skip = cluster_should_skip(p.status, 2 * p.splits);
   tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem_base;
   if (skip) {
-    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 2 * TN);
     return;
   }
 
@@ -135,15 +201,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
         tile_coords(tile, p.tiles_r, p.tiles_c, tr, tc, b);
         // Every other tile of a pair walks the reduction backwards: its first k-blocks are the ones the tile before
         // it (same row panels, as a rule) touched last, which are the ones still in L2.  The sum does not care.
-        for (int i = 0; i < nkb; ++i, ++idx) {
-          const int kb = (local & 1) ? nkb - 1 - i : i;
+        for (int i = 0; i < nks; ++i, ++idx) {
+          const int ks = ks0 + ((local & 1) ? nks - 1 - i : i);
           const int s = idx % C::NSTAGE;
           const uint32_t ph = (idx / C::NSTAGE) & 1;
           if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, actx, kErrGemmEmpty)) { ok = false; break; }
-          const uint32_t leader_full = map_to_cta(bar_full + 8 * s, 0);
+          const uint32_t leader_full = map_to_cta(bar_full + 8 * s, crank & ~1u);
           mbar_arrive_expect_tx_cluster(leader_full, C::XB + C::YB);
-          tma_load_3d_pair(sX + s * C::XB, &tm_x, leader_full, kb * bk, tr * C::TILE + (int)rank * C::BM, b);
-          tma_load_3d_pair(sY + s * C::YB, &tm_y, leader_full, kb * bk, tc * C::TILE + (int)rank * C::BNH, b);
+#pragma unroll
+          for (int h = 0; h < C::KSUB; ++h) {       // a k-block behind the end of K is zero-filled
+            const int k = (ks * C::KSUB + h) * bk;
+            tma_load_3d_pair(sX + s * C::XB + h * C::XSUB, &tm_x, leader_full, k, tr * C::TM + (int)rank * C::BM, b);
+            tma_load_3d_pair(sY + s * C::YB + h * C::YSUB, &tm_y, leader_full, k, tc * TN + (int)rank * C::BNH, b);
+          }
         }
       }
     }
@@ -151,10 +221,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
     // UMMA issue: all 32 lanes of the leader's warp run the loop, one elected lane executes the instructions
     if (rank == 0) {
       const uint32_t leader = elect_one();
-      const uint32_t peer_delta = map_to_cta(sBar, 1) - sBar;
-      constexpr uint32_t idesc_f16 = make_idesc(1, kFmtF16, kFmtF16, 0, 0, C::TILE, C::TILE);
-      constexpr uint32_t idesc_bf16 = make_idesc(1, kFmtBF16, kFmtBF16, 0, 0, C::TILE, C::TILE);
-      constexpr uint32_t idesc_tf32 = make_idesc(1, 2u, 2u, 0, 0, C::TILE, C::TILE);   // kind::tf32: format code 2
+      const uint16_t pair_mask = (uint16_t)(3u << (crank & ~1u));
+      constexpr uint32_t idesc_f16 = make_idesc(1, kFmtF16, kFmtF16, 0, 0, C::TM, TN);
+      constexpr uint32_t idesc_bf16 = make_idesc(1, kFmtBF16, kFmtBF16, 0, 0, C::TM, TN);
+      constexpr uint32_t idesc_tf32 = make_idesc(1, 2u, 2u, 0, 0, C::TM, TN);   // kind::tf32: format code 2
       const uint32_t idesc = p.tf32 ? idesc_tf32 : (p.bf16 ? idesc_bf16 : idesc_f16);
       int idx = 0, local = 0;
       bool ok = true;
@@ -163,30 +233,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
         const uint32_t acc_ph = (local >> 1) & 1;
         if (!mbar_wait_warp(bar_acc_empty + 8 * buf, acc_ph ^ 1u, actx, kErrGemmAccEmpty)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d = tmem_base + buf * 256;
-        for (int kb = 0; kb < nkb; ++kb, ++idx) {
+        const uint32_t d = tmem_base + buf * TN;
+        for (int ks = 0; ks < nks; ++ks, ++idx) {
           const int s = idx % C::NSTAGE;
           if (!mbar_wait_warp(bar_full + 8 * s, (idx / C::NSTAGE) & 1, actx, kErrGemmFull)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint64_t a0 = make_smem_desc(sX + s * C::XB, 16, 1024, kSwizzle128B);
-          const uint64_t b0 = make_smem_desc(sY + s * C::YB, 16, 1024, kSwizzle128B);
-          if (p.tf32) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)   // 32 bytes of reduction per UMMA: 8 tf32 elements
-              umma_ss_pair_tf32(d, desc_advance(a0, kk * 32), desc_advance(b0, kk * 32), idesc, (kb | kk) != 0 ? 1u : 0u, leader);
-          } else {
+          for (int h = 0; h < C::KSUB; ++h) {
+            const uint64_t a0 = make_smem_desc(sX + s * C::XB + h * C::XSUB, 16, 1024, kSwizzle128B);
+            const uint64_t b0 = make_smem_desc(sY + s * C::YB + h * C::YSUB, 16, 1024, kSwizzle128B);
+            if (p.tf32) {
 #pragma unroll
-            for (int kk = 0; kk < C::BK / 16; ++kk)
-              umma_ss_e<false, true>(d, desc_advance(a0, kk * 32), desc_advance(b0, kk * 32), idesc,
-                                     (kb | kk) != 0 ? 1u : 0u, leader);
+              for (int kk = 0; kk < 4; ++kk)   // 32 bytes of reduction per UMMA: 8 tf32 elements
+                umma_ss_pair_tf32(d, desc_advance(a0, kk * 32), desc_advance(b0, kk * 32), idesc, (ks | h | kk) != 0 ? 1u : 0u,
+                                  leader);
+            } else {
+#pragma unroll
+              for (int kk = 0; kk < C::BK / 16; ++kk)
+                umma_ss_e<false, true>(d, desc_advance(a0, kk * 32), desc_advance(b0, kk * 32), idesc,
+                                       (ks | h | kk) != 0 ? 1u : 0u, leader);
+            }
           }
-          umma_commit_e<true>(bar_empty + 8 * s, leader);                // this CTA's stage
-          umma_commit_e<true>(bar_empty + 8 * s + peer_delta, leader);   // the peer's stage
+          umma_commit_pair_e(bar_empty + 8 * s, pair_mask, leader);      // the stage is free in both CTAs
         }
-        if (ok) {
-          umma_commit_e<true>(bar_acc_full + 8 * buf, leader);
-          umma_commit_e<true>(bar_acc_full + 8 * buf + peer_delta, leader);
-        }
+        if (ok) umma_commit_pair_e(bar_acc_full + 8 * buf, pair_mask, leader);
       }
     }
   } else {
@@ -198,11 +268,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
     const int r = q * 32 + lane;                       // row within this CTA's 128 rows
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     const int row_in_tile = (int)rank * C::BM + r;
-    const uint32_t leader_acc_empty = map_to_cta(bar_acc_empty, 0);
+    const uint32_t leader_acc_empty = map_to_cta(bar_acc_empty, crank & ~1u);
     const int esz = p.tf32 ? 4 : 2;
     const int ccols = 128 / esz;                       // columns per chunk
-    const int nchunk = C::TILE / ccols;
+    const int nchunk = TN / ccols;
     const bool storer = (warp == 2 && lane == 0);
+    if (p.direct) {          // hand-over: the units other pairs will finish, [unit][4 columns][row][16 bytes]
+      if (mbar_wait_warp(bar_acc_full, 0, actx, kErrGemmAccFull)) {
+        tc_fence_after_sync();
+        for (int u = 0; u < C::UNITS; ++u) {
+          if (u % p.splits == part) continue;
+          uint32_t acc[32];
+          tmem_ld_x32(tmem_base + lane_base + u * 32, acc);
+          tmem_wait_ld();
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sX + u * C::UNITB + g * 2048 + r * 16),
+                         "r"(acc[4 * g]), "r"(acc[4 * g + 1]), "r"(acc[4 * g + 2]), "r"(acc[4 * g + 3]) : "memory");
+        }
+      }
+    } else {
     int local = 0;
     uint32_t n = 0;                                    // chunks staged so far: chunk n uses staging tile n & 1
     bool ok = true;
@@ -210,12 +295,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
       int tr, tc, b;
       tile_coords(tile, p.tiles_r, p.tiles_c, tr, tc, b);
       const int buf = local & 1;
+      const int row = tr * C::TM + row_in_tile;
+      const int col0 = tc * TN;
+      const size_t src_at = (size_t)b * p.d_batch + (size_t)row * p.ldd + col0;
+      const bool with_src = p.beta != 0.f && row < p.R;
+      SourceRow src;
+      if (with_src) load_source(src, p, src_at, p.Cn - col0);     // the first 32 columns, while the tile is being computed
       ok = mbar_wait_warp(bar_acc_full + 8 * buf, (local >> 1) & 1, actx, kErrGemmAccFull);
       if (!ok) break;
       tc_fence_after_sync();
-      const int row = tr * C::TILE + row_in_tile;
-      const int col0 = tc * C::TILE;
-      const size_t src_row = (size_t)b * p.d_batch + (size_t)row * p.ldd;
 #pragma unroll 1
       for (int ch = 0; ch < nchunk; ++ch, ++n) {
         const uint32_t sb = n & 1u;
@@ -229,46 +317,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
         for (int h = 0; h < ccols / 32; ++h) {         // 32 accumulator columns at a time
           uint32_t acc[32];
           const int cbase = ch * ccols + h * 32;       // first of these columns within the tile
-          tmem_ld_x32(tmem_base + lane_base + buf * 256 + cbase, acc);
+          tmem_ld_x32(tmem_base + lane_base + buf * TN + cbase, acc);
           tmem_wait_ld();
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = p.alpha * __uint_as_float(acc[i]);
-          if (p.beta != 0.f && row < p.R) {            // the source matrix: this thread's row, straight from global memory
-            if (p.tf32) {
-              const float* srow = reinterpret_cast<const float*>(p.src) + src_row + col0 + cbase;
-#pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                if (col0 + cbase + g * 4 < p.Cn) {
-                  const float4 old = *reinterpret_cast<const float4*>(srow + g * 4);
-                  v[g * 4] += p.beta * old.x; v[g * 4 + 1] += p.beta * old.y;
-                  v[g * 4 + 2] += p.beta * old.z; v[g * 4 + 3] += p.beta * old.w;
-                }
-              }
-            } else {
-              const uint16_t* srow = reinterpret_cast<const uint16_t*>(p.src) + src_row + col0 + cbase;
-#pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                if (col0 + cbase + g * 8 < p.Cn) {
-                  const uint4 old = *reinterpret_cast<const uint4*>(srow + g * 8);
-                  const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) {
-                    float lo, hi;
-                    if (p.bf16) {
-                      lo = __uint_as_float(ow[i] << 16);
-                      hi = __uint_as_float(ow[i] & 0xffff0000u);
-                    } else {
-                      const __half2 hh = *reinterpret_cast<const __half2*>(&ow[i]);
-                      lo = __low2float(hh);
-                      hi = __high2float(hh);
-                    }
-                    v[g * 8 + 2 * i] += p.beta * lo;
-                    v[g * 8 + 2 * i + 1] += p.beta * hi;
-                  }
-                }
-              }
-            }
+          if (with_src) {
+            const SourceRow cur = src;
+            if (cbase + 32 < TN) load_source(src, p, src_at + cbase + 32, p.Cn - (col0 + cbase + 32));
+            add_source(v, p, cur);
           }
           // 16-byte pieces of the row, piece index XOR (row & 7): the 128-byte swizzle the TMA store undoes
           if (p.tf32) {
@@ -282,14 +339,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
           } else {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-              uint32_t w0, w1, w2, w3;
-              if (p.bf16) {
-                w0 = pack_bf16x2(v[g * 8], v[g * 8 + 1]); w1 = pack_bf16x2(v[g * 8 + 2], v[g * 8 + 3]);
-                w2 = pack_bf16x2(v[g * 8 + 4], v[g * 8 + 5]); w3 = pack_bf16x2(v[g * 8 + 6], v[g * 8 + 7]);
-              } else {
-                w0 = pack_f16x2(v[g * 8], v[g * 8 + 1]); w1 = pack_f16x2(v[g * 8 + 2], v[g * 8 + 3]);
-                w2 = pack_f16x2(v[g * 8 + 4], v[g * 8 + 5]); w3 = pack_f16x2(v[g * 8 + 6], v[g * 8 + 7]);
-              }
+              const uint32_t w0 = pack_out(p.bf16, v[g * 8], v[g * 8 + 1]), w1 = pack_out(p.bf16, v[g * 8 + 2], v[g * 8 + 3]);
+              const uint32_t w2 = pack_out(p.bf16, v[g * 8 + 4], v[g * 8 + 5]), w3 = pack_out(p.bf16, v[g * 8 + 6], v[g * 8 + 7]);
               const uint32_t piece = (uint32_t)(h * 4 + g) ^ (uint32_t)(r & 7);
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_addr + piece * 16), "r"(w0), "r"(w1),
                            "r"(w2), "r"(w3) : "memory");
@@ -305,7 +356,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
         if (storer) {
           if (!mbar_wait(bar_staged + 8 * sb, (n >> 1) & 1u, actx, kErrGemmStaged)) { ok = false; }
           else {
-            tma_store_3d(&tm_d, stage, col0 + ch * ccols, tr * C::TILE + (int)rank * C::BM, b);
+            tma_store_3d(&tm_d, stage, col0 + ch * ccols, tr * C::TM + (int)rank * C::BM, b);
             tma_store_commit();
             tma_store_wait_read1();            // every store but this one has read its staging tile
             if (n >= 1u) mbar_arrive(bar_stage_free + 8 * (sb ^ 1u));
@@ -316,6 +367,93 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
       }
     }
     if (storer) tma_store_wait_read0();
+    }
+  }
+
+  if (p.direct) {
+    __syncwarp();
+    cluster_sync_all();      // every CTA's accumulator is in its shared memory
+    if (warp >= 2 && !*s_abort) {
+      const int q = warp & 3, r = q * 32 + lane;
+      int tr, tc, b;
+      tile_coords(pair_id, p.tiles_r, p.tiles_c, tr, tc, b);
+      const int row = tr * C::TM + (int)rank * C::BM + r;
+      for (int u = part; u < C::UNITS; u += p.splits) {
+        const int col = tc * TN + u * 32;
+        if (col >= p.Cn) break;
+        const size_t at_row = (size_t)b * p.d_batch + (size_t)row * p.ldd + col;
+        SourceRow src;
+        if (p.beta != 0.f && !p.trans && row < p.R) load_source(src, p, at_row, p.Cn - col);
+        uint32_t acc[32];
+        tmem_ld_x32(tmem_base + ((uint32_t)(q * 32) << 16) + u * 32, acc);
+        tmem_wait_ld();
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = 0.f;
+        for (int o = 0; o < p.splits; ++o) {           // in the order of the reduction
+          if (o == part) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(acc[i]);
+            continue;
+          }
+          const uint32_t at = map_to_cta(sX + u * C::UNITB + r * 16, (uint32_t)(2 * o) + rank);
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const float4 x = ld_shared_cluster_f32x4(at + g * 2048);
+            v[4 * g] += x.x; v[4 * g + 1] += x.y; v[4 * g + 2] += x.z; v[4 * g + 3] += x.w;
+          }
+        }
+        if (row < p.R) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
+          if (p.trans) {       // the warp's 32 rows are neighbours in D
+            const size_t at = (size_t)b * p.d_batch + (size_t)col * p.ldd + row;
+            if (p.beta != 0.f) {                       // all reads ahead of the first write, which might be to the same matrix
+              float old[32];
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                old[i] = 0.f;
+                if (col + i < p.Cn) {
+                  if (p.tf32) {
+                    old[i] = reinterpret_cast<const float*>(p.src)[at + (size_t)i * p.ldd];
+                  } else {
+                    const uint16_t h = reinterpret_cast<const uint16_t*>(p.src)[at + (size_t)i * p.ldd];
+                    old[i] = p.bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h));
+                  }
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] += p.beta * old[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (col + i < p.Cn) {
+                if (p.tf32) reinterpret_cast<float*>(p.d)[at + (size_t)i * p.ldd] = v[i];
+                else reinterpret_cast<uint16_t*>(p.d)[at + (size_t)i * p.ldd] = (uint16_t)(pack_out(p.bf16, v[i], 0.f) & 0xffffu);
+              }
+            }
+          } else {
+            if (p.beta != 0.f) add_source(v, p, src);
+            if (p.tf32) {
+              float* dst = reinterpret_cast<float*>(p.d) + at_row;
+#pragma unroll
+              for (int g = 0; g < 8; ++g)
+                if (col + g * 4 < p.Cn)
+                  *reinterpret_cast<float4*>(dst + g * 4) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            } else {
+              uint16_t* dst = reinterpret_cast<uint16_t*>(p.d) + at_row;
+#pragma unroll
+              for (int g = 0; g < 4; ++g)
+                if (col + g * 8 < p.Cn)
+                  *reinterpret_cast<uint4*>(dst + g * 8) =
+                      make_uint4(pack_out(p.bf16, v[g * 8], v[g * 8 + 1]), pack_out(p.bf16, v[g * 8 + 2], v[g * 8 + 3]),
+                                 pack_out(p.bf16, v[g * 8 + 4], v[g * 8 + 5]), pack_out(p.bf16, v[g * 8 + 6], v[g * 8 + 7]));
+            }
+          }
+        }
+        __syncwarp();        // the next unit's tcgen05.ld takes the whole warp
+      }
+    }
   }
 
   settle_if_aborted(s_abort);
@@ -324,8 +462,102 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   cluster_sync_all();           // no CTA leaves while its peer may still read its shared memory or signal it
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc_pair(tmem_base, 512);
+    tmem_dealloc_pair(tmem_base, 2 * TN);
   }
+}
+
+struct GemmPlan { int tn, splits, trans; };
+
+// Clusters of 2 * splits CTAs (splits = 1..4) that can be resident at once on the current device, by the largest kernel.
+static const int* resident_clusters() {   // [splits]
+  static thread_local int of_dev = -1;
+  static thread_local int n[5];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  if (of_dev != dev) {
+    for (int s = 1; s <= 4; ++s) {
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = (unsigned)(2 * s);
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(2 * s) * 256);
+      cfg.blockDim = dim3(GemmCfg<256>::NTHREADS);
+      cfg.dynamicSmemBytes = GemmCfg<256>::SMEM_BYTES;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      n[s] = 0;
+      if (cudaFuncSetAttribute(gemm_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<256>::SMEM_BYTES) !=
+              cudaSuccess || cudaOccupancyMaxActiveClusters(&n[s], gemm_kernel<256>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n[s] = 0;
+      }
+    }
+    of_dev = dev;
+  }
+  return n;
+}
+
+// Tile width, split and orientation.  With two waves of 256 x 256 tiles or more, and whenever nothing else is estimated to
+// be faster, 256 without a split.  Below that SMs stand idle, and the estimate decides, in us: a fixed part (launch, first
+// loads, epilogue), a time per k-block of the longest chain of tiles (a narrower tile costs less, but not in proportion; rows
+// whose pitch is not a multiple of 32 bytes make TMA fetch every sector's neighbour too), the exchange of a split, and for
+// exchanged operands, which pay where D has few rows, the two-byte stores of each column a CTA finishes.  The constants are
+// fits to a sweep of 24 shapes x 2 orders x 18 plans in bf16 and fp32; the plan it chose was the fastest or within 5 % of it
+// for nearly all.  us before / after, bf16: 2048 x 768 x 4096 25.4 / 16.4, 16 x 3088 x 9968 50.4 / 12.8, 1408 x 536 x 2816
+// 19.3 / 11.2, 88 x 88 x 80 6.9 / 5.2.
+static GemmPlan plan_gemm(int R, int Cn, int K, int L, bool fp32) {
+  const int* resident = resident_clusters();
+  const int pairs = resident ? resident[1] : 0;
+  GemmPlan best = {256, 1, 0};
+  auto tiles_of = [&](int rows, int cols, int tn) { return (long long)((rows + 255) / 256) * ((cols + tn - 1) / tn) * L; };
+  if (pairs <= 0 || tiles_of(R, Cn, 256) > 2 * pairs) return best;
+  const long long pitch = (long long)K * (fp32 ? 4 : 2);
+  const int nkb = (int)((pitch + 127) / 128);
+  const bool pitch32 = pitch % 32 == 0;
+  static const float fixed[3] = {6.3f, 5.3f, 4.8f};
+  static const float per_kb[2][3] = {{0.37f, 0.33f, 0.29f}, {0.30f, 0.17f, 0.15f}};
+  static const float exchange[3][5] = {{0, 0, 2.8f, 3.5f, 4.4f}, {0, 0, 1.9f, 2.4f, 3.0f}, {0, 0, 1.4f, 2.1f, 2.4f}};
+  float best_t = 0.f;
+  for (int trans = 0; trans < 2; ++trans)
+    for (int w = 0; w < 3; ++w)
+      for (int s = 1; s <= 4; ++s) {
+        const int tn = 256 >> w, stages = (nkb + (w ? 1 : 0)) / (w ? 2 : 1);
+        const long long tiles = trans ? tiles_of(Cn, R, tn) : tiles_of(R, Cn, tn);
+        if (s > stages || ((s > 1 || trans) && tiles > resident[s])) continue;
+        const long long waves = (tiles + pairs - 1) / pairs;
+        float t = fixed[w] + per_kb[pitch32][w] * (float)((nkb + s - 1) / s) * (float)waves + exchange[w][s];
+        if (trans) t += 0.3f + 0.03f * (float)(R < tn ? R : tn) / (float)s;
+        if (best_t == 0.f || t < best_t) { best_t = t; best = GemmPlan{tn, s, trans}; }
+      }
+  return best;
+}
+
+template <int TN>
+static int launch_gemm(const CUtensorMap& tm_x, const CUtensorMap& tm_y, const CUtensorMap& tm_d, const GemmParams& p,
+                       int iterations, cudaStream_t stream) {
+  using C = GemmCfg<TN>;
+  static thread_local int attr_dev = -1;
+  static thread_local int sm_count = 0;
+  int dev = 0;
+  if (note_cuda(cudaGetDevice(&dev), "cudaGetDevice") != cudaSuccess) return CFK_ERR_NO_DRIVER;
+  if (attr_dev != dev) {
+    if (note_cuda(cudaFuncSetAttribute(gemm_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES),
+                  "cudaFuncSetAttribute(gemm smem)") != cudaSuccess)
+      return CFK_ERR_LAUNCH;
+    if (note_cuda(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev), "sm count") != cudaSuccess)
+      return CFK_ERR_LAUNCH;
+    attr_dev = dev;
+  }
+  const long long total = (long long)p.tiles_r * p.tiles_c * p.L;
+  // the pairs (one per two SMs) are persistent and walk the tiles, or there is a cluster per tile
+  const long long clusters = p.direct || total < sm_count / 2 ? total : sm_count / 2;
+  const dim3 grid((unsigned)(2 * p.splits * clusters));
+  for (int it = 0; it < iterations; ++it)
+    if (note_cuda(launch_overlapped_in(2 * p.splits, gemm_kernel<TN>, grid, dim3(C::NTHREADS), C::SMEM_BYTES, stream, tm_x, tm_y,
+                                       tm_d, p), "gemm launch") != cudaSuccess)
+      return CFK_ERR_LAUNCH;
+  return CFK_OK;
 }
 
 }  // namespace cfk
@@ -347,62 +579,53 @@ extern "C" int cfk_gemm(const cfk_gemm_args* a, cfk_stream_t stream) {
   // the swapped product.
   const void* x = a->c_row_major ? a->a : a->b;
   const void* y = a->c_row_major ? a->b : a->a;
-  const int R = a->c_row_major ? a->m : a->n;
-  const int Cn = a->c_row_major ? a->n : a->m;
+  int R = a->c_row_major ? a->m : a->n;
+  int Cn = a->c_row_major ? a->n : a->m;
 
-  CUtensorMap tm_x, tm_y;
+  const GemmPlan plan = plan_gemm(R, Cn, a->k, a->l, a->dtype == CFK_FP32);
+
+  CUtensorMap tm_x, tm_y, tm_d;
   const uint64_t esz = (uint64_t)dtype_size(a->dtype);
   const uint32_t bk = (uint32_t)(128 / esz);                   // one 128-byte span of the reduction per stage
-  const uint64_t xd[3] = {(uint64_t)a->k, (uint64_t)R, (uint64_t)a->l};
-  const uint64_t xs[2] = {(uint64_t)a->k * esz, (uint64_t)a->k * esz * (uint64_t)R};
-  const uint32_t xb[3] = {bk, GemmCfg::BM, 1};                 // per CTA: 128 rows of X
-  const uint64_t yd[3] = {(uint64_t)a->k, (uint64_t)Cn, (uint64_t)a->l};
-  const uint64_t ys[2] = {(uint64_t)a->k * esz, (uint64_t)a->k * esz * (uint64_t)Cn};
-  const uint32_t yb[3] = {bk, GemmCfg::BNH, 1};                // per CTA: 128 rows of Y
   int rc;
-  if ((rc = encode_tiled(&tm_x, a->dtype, 3, x, xd, xs, xb, 128))) return rc;
-  if ((rc = encode_tiled(&tm_y, a->dtype, 3, y, yd, ys, yb, 128))) return rc;
+  auto operand = [&](CUtensorMap* tm, const void* base, int rows, int box_rows) {
+    const uint64_t d[3] = {(uint64_t)a->k, (uint64_t)rows, (uint64_t)a->l};
+    const uint64_t st[2] = {(uint64_t)a->k * esz, (uint64_t)a->k * esz * (uint64_t)rows};
+    const uint32_t box[3] = {bk, (uint32_t)box_rows, 1};
+    return encode_tiled(tm, a->dtype, 3, base, d, st, box, 128);
+  };
+  // per CTA: 128 rows of X, and half the columns of a tile in rows of Y; `trans` exchanges the two
+  if ((rc = operand(plan.trans ? &tm_y : &tm_x, x, R, plan.trans ? plan.tn / 2 : 128))) return rc;
+  if ((rc = operand(plan.trans ? &tm_x : &tm_y, y, Cn, plan.trans ? 128 : plan.tn / 2))) return rc;
 
   // D (row-major R x Cn per batch) for the TMA store of the epilogue: boxes of 128 rows x 128 bytes
-  CUtensorMap tm_d;
   const uint64_t dd[3] = {(uint64_t)Cn, (uint64_t)R, (uint64_t)a->l};
   const uint64_t ds[2] = {(uint64_t)Cn * esz, (uint64_t)Cn * esz * (uint64_t)R};
-  const uint32_t db[3] = {bk, GemmCfg::BM, 1};
+  const uint32_t db[3] = {bk, 128, 1};
   if ((rc = encode_tiled(&tm_d, a->dtype, 3, a->c, dd, ds, db, 128))) return rc;
 
+  if ((long long)((R + 255) / 256) * ((Cn + 255) / 256) * a->l > 0x7fffffffLL) return CFK_ERR_UNSUPPORTED;
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
-  p.R = R; p.Cn = Cn; p.K = a->k; p.L = a->l;
   p.ldd = Cn;
   p.d_batch = (int64_t)R * Cn;
+  if (plan.trans) std::swap(R, Cn);
+  p.R = R; p.Cn = Cn; p.K = a->k; p.L = a->l;
+  p.trans = plan.trans;
+  p.direct = plan.splits > 1 || plan.trans;
   p.d = a->c;
   p.src = a->c_src ? a->c_src : a->c;
   p.alpha = a->alpha; p.beta = a->beta;
   p.bf16 = a->dtype == CFK_BF16;
   p.tf32 = a->dtype == CFK_FP32;
-  p.tiles_r = (R + GemmCfg::TILE - 1) / GemmCfg::TILE;
-  p.tiles_c = (Cn + GemmCfg::TILE - 1) / GemmCfg::TILE;
+  p.tiles_r = (R + 255) / 256;
+  p.tiles_c = (Cn + plan.tn - 1) / plan.tn;
+  p.splits = plan.splits;
   p.status = status;
 
-  static thread_local int attr_dev = -1;
-  static thread_local int sm_count = 0;
-  int dev = 0;
-  if (note_cuda(cudaGetDevice(&dev), "cudaGetDevice") != cudaSuccess) return CFK_ERR_NO_DRIVER;
-  if (attr_dev != dev) {
-    if (note_cuda(cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg::SMEM_BYTES),
-                  "cudaFuncSetAttribute(gemm smem)") != cudaSuccess)
-      return CFK_ERR_LAUNCH;
-    if (note_cuda(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev), "sm count") != cudaSuccess)
-      return CFK_ERR_LAUNCH;
-    attr_dev = dev;
+  switch (plan.tn) {
+    case 256: return launch_gemm<256>(tm_x, tm_y, tm_d, p, a->iterations, (cudaStream_t)stream);
+    case 128: return launch_gemm<128>(tm_x, tm_y, tm_d, p, a->iterations, (cudaStream_t)stream);
+    default: return launch_gemm<64>(tm_x, tm_y, tm_d, p, a->iterations, (cudaStream_t)stream);
   }
-  const long long total = (long long)p.tiles_r * p.tiles_c * p.L;
-  if (total > 0x7fffffffLL) return CFK_ERR_UNSUPPORTED;
-  const long long pairs = total < sm_count / 2 ? total : sm_count / 2;   // one CTA pair per two SMs
-  const int grid = (int)(2 * pairs);
-  for (int it = 0; it < a->iterations; ++it)
-    if (note_cuda(launch_overlapped(gemm_kernel, grid, GemmCfg::NTHREADS, GemmCfg::SMEM_BYTES, (cudaStream_t)stream, tm_x, tm_y,
-                                    tm_d, p), "gemm launch") != cudaSuccess)
-      return CFK_ERR_LAUNCH;
-  return CFK_OK;
 }

@@ -1,0 +1,54 @@
+"""GEMM shapes with too few 256 x 256 tiles for the SMs: narrower tiles, the reduction split over a cluster, operands
+exchanged.  The sizes are the smallest found for each of the plans (ragged in every dimension, last k-blocks that are mostly
+zero fill, columns no pair has to finish, batches); the truth is the CPU oracle, and for fp32 the fp64 product of the operands
+cut to tf32.  Tolerance: half a unit of the output type (test_gemm_gpu.py) plus fp32 summation order, which for K products of
+size up to 1 stays below K * 2^-24 * sqrt(K) / 2."""
+import numpy as np
+import pytest
+import torch
+
+from test_gemm_gpu import run
+
+pytestmark = pytest.mark.gpu
+
+# (M, N, K, L, row-major): tile width / split / operands exchanged, in bf16
+SHAPES = [(8, 8, 8, 1, False),            # 64
+          (8, 1544, 72, 3, True),         # 64, exchanged
+          (8, 1544, 1032, 1, True),       # 64 / 2
+          (8, 2056, 1032, 3, True),       # 64 / 2, exchanged
+          (8, 8, 1032, 1, False),         # 64 / 3: column units without an owner
+          (8, 1544, 1032, 3, True),       # 64 / 3, exchanged
+          (8, 8, 2056, 1, False),         # 64 / 4
+          (8, 2056, 1032, 1, True),       # 64 / 4, exchanged
+          (16, 1544, 72, 3, True),        # 128
+          (136, 776, 2056, 3, False),     # 128 / 2
+          (72, 2056, 2056, 3, True),      # 128 / 2, exchanged
+          (72, 776, 1032, 3, True),       # 128 / 3
+          (72, 520, 4104, 3, True),       # 128 / 4
+          (1032, 72, 2056, 3, False),     # 128 / 4, exchanged
+          (264, 776, 2056, 3, True),      # 256 / 2
+          (264, 2056, 2056, 1, True),     # 256 / 3
+          (1032, 520, 4104, 1, False)]    # 256 / 4
+
+
+@pytest.mark.parametrize("M,N,K,L,row_major", SHAPES)
+def test_narrow_and_split_plans_match_the_oracle(lib, oracle, cuda, M, N, K, L, row_major):
+    run(lib, oracle, M, N, K, dtype=0, row_major=row_major, L=L, seed=K)
+    run(lib, oracle, M, N, K, dtype=1, row_major=row_major, L=L, alpha=0.5, beta=2.0, seed=K + 1)
+    run(lib, oracle, M, N, K, dtype=0, row_major=not row_major, L=L, alpha=-1.0, beta=0.5, seed=K + 2)
+
+
+@pytest.mark.parametrize("M,N,K,L,row_major", SHAPES)
+def test_narrow_and_split_plans_in_tf32_with_a_separate_source(lib, cuda, M, N, K, L, row_major):
+    g = torch.Generator().manual_seed(M + N)
+    a, b = (torch.rand(L, r, K, generator=g) * 2 - 1 for r in (M, N))
+    shape = (L, M, N) if row_major else (L, N, M)
+    src = torch.rand(*shape, generator=g)
+    d = torch.full((L * M * N + 64,), -3.0, device="cuda")
+    lib.gemm(a.cuda(), b.cuda(), d, dtype=3, m=M, n=N, k=K, l=L, alpha=0.5, beta=-2.0, c_row_major=row_major, c_src=src.cuda())
+    lib.check_device()
+    cut = lambda x: x.view(torch.int32).bitwise_and(-8192).view(torch.float32).double().numpy()    # noqa: E731
+    ref = 0.5 * np.einsum("lmk,lnk->lmn" if row_major else "lmk,lnk->lnm", cut(a), cut(b), optimize=True) - 2.0 * src.double().numpy()
+    err = np.abs(d[:L * M * N].view(*shape).cpu().numpy() - ref).max()
+    assert err <= K * 2.0 ** -24 * K ** 0.5 / 2 + 2.0 ** -22, err
+    assert bool((d[L * M * N:] == -3.0).all())
