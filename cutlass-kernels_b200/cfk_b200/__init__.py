@@ -109,7 +109,7 @@ class CfkLib:
     # -- conveniences ---------------------------------------------------------------------------
     # A call of a few microseconds on the device is bound by the host, so the structs are filled by one constructor call
     # each, packed strides share a zero array, and the wrappers name their arguments instead of passing dicts on
-    # (argument handling of fmha_forward 6.4 -> 3.2 us, of gemm 2.9 -> 1.7).
+    # (attention 1 x 2 x 128 x 128: 9.3 -> 6.7 us a call).
     def fmha_args(self, q, k, v, o, *, dtype, batch, heads, seqlen_q, seqlen_kv, head_dim, softmax_scale,
                   causal=False, out_dtype=FP16, p_split_keys=-1, lse=None, mi=None, sprime=None,
                   q_descale=1.0, k_descale=1.0, v_descale=1.0, iterations=1,

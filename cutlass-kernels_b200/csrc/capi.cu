@@ -248,6 +248,51 @@ static int decode_splits(long long groups, int ntiles, int resident) {
   return s;
 }
 
+// One 128-row tile per CTA, two CTAs per SM (fmha_fwd_tile_sm100.cuh), against one 256-row block per SM
+// (fmha_fwd_sm100.cuh).  Returns the number of CTAs that share a tile's keys, 0 for the 256-row kernel.
+//   Fewer tiles than CTAs fit on the chip, and at least 8 key tiles: the keys are split as far as the chip has room, two key
+//   tiles per CTA at least, eight where there is room for two parts only (8 heads, 1024 x 1024 in two: 18.4 against 17.0).  us, bf16 d = 128 causal, 256-row kernel / whole keys / split: 8 heads, 256 x 2048 28.4 / 25.4 /
+//   13.7 (8 parts), 512 x 4096 51.2 / 46.3 / 18.8 (8), 2048 x 2048 29.0 / 28.2 / 25.9 (2); 24 heads, 512 x 4096 52.1 / 51.6 /
+//   40.9 (2).
+//   Otherwise short keys, up to 12 tiles: the estimate below decides, with 6 % in favour of the 256-row kernel.  300 heads,
+//   128 x 128 18.0 / 12.3, 300 x 300 48.4 / 33.7; 100 heads, 640 x 640 34.2 / 24.4.  With longer keys the 256-row kernel, which
+//   reads K and V once per 256 rows, is as fast or faster: 8 heads, 8192 x 8192 107.5 / 120.0.
+// The estimate, in us: a fixed time per CTA, a time per key tile, and for causal calls the tail of the heaviest-first order;
+// the constants are fits to a sweep of 24 shapes x causal or not for each type (root mean square error 6-13 %).
+struct TileCost { float fixed, per_tile, tail, offset; };
+static float estimate_us(const cfk_fmha_args* a, int rows, int slots, const TileCost& c) {
+  const int nq = (a->seqlen_q + rows - 1) / rows, nall = (a->seqlen_kv + 127) / 128;
+  const long long bh = (long long)a->batch * a->heads, units = bh * nq;
+  auto tiles_of = [&](int q) {
+    const int nc = (int)(((long long)q * rows + rows - 1 + a->seqlen_kv - a->seqlen_q) / 128 + 1);
+    return a->causal && nc < nall ? nc : nall;
+  };
+  const float longest = c.fixed + c.per_tile * (float)tiles_of(nq - 1);
+  if (units <= slots) return longest + c.offset;
+  if (!a->causal || nq == 1) return ceilf((float)units / (float)slots - 0.02f) * longest + c.offset;
+  float sum = 0.f;
+  for (int q = 0; q < nq; ++q) sum += c.fixed + c.per_tile * (float)tiles_of(q);
+  const float t = sum * (float)bh / (float)slots + c.tail * (c.fixed + c.per_tile * (float)tiles_of(0));
+  return (t > longest ? t : longest) + c.offset;
+}
+static int tile_plan(const cfk_fmha_args* a) {
+  constexpr int kSMs = 148;
+  const long long units = (long long)a->batch * a->heads * ((a->seqlen_q + 127) / 128);
+  const int nall = (a->seqlen_kv + 127) / 128;
+  if (nall >= 8 && 2 * units <= 2 * kSMs) {
+    int s = 2;
+    while (s < 8 && units * 2 * s <= 2 * kSMs && nall >= 4 * s) s *= 2;
+    if (s > 2 || nall >= 16) return s;
+  }
+  if (nall > 12 || units > 0x7fffffffLL) return 0;
+  static const TileCost block256[2][2] = {{{4.31f, 1.33f, 0.86f, 1.45f}, {6.33f, 1.50f, 0.88f, 1.11f}},
+                                          {{3.04f, 1.38f, 0.83f, 1.13f}, {4.17f, 1.37f, 0.76f, 0.64f}}};
+  static const TileCost tile128[2][2] = {{{4.60f, 1.20f, 1.09f, 1.91f}, {7.11f, 1.49f, 0.99f, 1.33f}},
+                                         {{3.33f, 1.20f, 0.83f, 1.86f}, {4.40f, 1.25f, 0.71f, 1.66f}}};   // [e4m3][d = 128]
+  const int e = a->dtype == CFK_E4M3 && !a->v_fp16, d = a->head_dim == 128;
+  return estimate_us(a, 128, 2 * kSMs, tile128[e][d]) < 0.94f * estimate_us(a, 256, kSMs, block256[e][d]) ? 1 : 0;
+}
+
 // Argument checks, TMA descriptors, kernel parameters and kernel choice of one FMHA call: everything of the launch
 // except the status pointer and the stream, which the two entry points supply (allocated block / static array).
 // *p_dtype receives the type P is rounded to (and V is stored in).
@@ -287,8 +332,13 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   if (L.variant == 1 && (a->dtype == CFK_E4M3 || a->head_dim != 128)) L.variant = 0;
   if (a->head_dim == 256) L.variant = 0;
   const long long groups16 = (long long)a->batch * a->heads * ((a->seqlen_q + 15) / 16);
-  const bool decode = L.variant == 0 && !a->s_dump && decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim);
+  // an explicit schedule asks for the kernel that has one
+  const int sched = g_tunable[CFK_TUNE_FMHA_SCHED].load();
+  const bool by_size = L.variant == 0 && sched < 0 && !a->s_dump;
+  const bool decode = by_size && decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim);
   if (decode) L.variant = 3;
+  const int tile_splits = by_size && !decode && a->head_dim != 256 ? tile_plan(a) : 0;
+  if (tile_splits > 0) L.variant = 4;
   const int q_rows = decode ? 16 : 128, kv_rows = decode ? decode_tile_keys(a->head_dim, dtype_size(vdt)) : 128;
   if ((rc = encode_bshd(&L.tm_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], q_rows)))
     return rc;
@@ -300,11 +350,12 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
     return rc;
   if ((rc = encode_bshd(&L.tm_o, a->out_dtype, a->o, a->batch, a->seqlen_q, a->heads, a->head_dim, os[0], os[1], os[2], 128)))
     return rc;
+  L.sp.o = a->o;
+  L.sp.o_b = os[0]; L.sp.o_s = os[1]; L.sp.o_h = os[2];
+  L.sp.splits = tile_splits;
   if (decode) {
-    L.dec.o = a->o;
-    L.dec.o_b = os[0]; L.dec.o_s = os[1]; L.dec.o_h = os[2];
-    L.dec.nqb = (a->seqlen_q + 15) / 16;
-    L.dec.splits = decode_splits(groups16, (a->seqlen_kv + kv_rows - 1) / kv_rows,
+    L.sp.nqb = (a->seqlen_q + 15) / 16;
+    L.sp.splits = decode_splits(groups16, (a->seqlen_kv + kv_rows - 1) / kv_rows,
                                  148 * decode_ctas_per_sm(a->head_dim, esz, dtype_size(vdt)));
   }
 
@@ -320,14 +371,13 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   p.B = a->batch; p.H = a->heads; p.Sq = a->seqlen_q; p.Skv = a->seqlen_kv;
   p.causal = a->causal ? 1 : 0;
   p.out_bf16 = a->out_dtype == CFK_BF16;
-  // one 128-row tile per CTA at head dimension 256 and in the persistent kernel, two side by side otherwise
-  p.nqblk = (a->head_dim == 256 || L.variant == 2) ? (a->seqlen_q + 127) / 128 : (a->seqlen_q + 255) / 256;
+  // one 128-row tile per CTA at head dimension 256 and in kernels 2 and 4, two side by side otherwise
+  p.nqblk = (a->head_dim == 256 || L.variant == 2 || L.variant == 4) ? (a->seqlen_q + 127) / 128 : (a->seqlen_q + 255) / 256;
   {
     // Default by input type, the measured best: with e4m3 Q and K the first GEMM is short enough for the two query
     // tiles to take turns on one score buffer (+8-12 % on every e4m3 shape together with the share of exponentials on
     // the FMA pipe that goes with it, below); with 16-bit inputs the hand-over of
     // the buffer would set the pace (c3 1246 -> 1221 TFLOP/s).
-    const int sched = g_tunable[CFK_TUNE_FMHA_SCHED].load();
     p.sched = sched < 0 ? (a->dtype == CFK_E4M3 ? 1 : 0) : sched;
   }
   p.split_keys = a->dtype == CFK_BF16 ? (a->p_split_keys < 0 ? 1024 : a->p_split_keys) : 0;
@@ -341,7 +391,7 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   // 16-bit at d = 256 (one softmax warpgroup, tensor-bound): none (fp16 1302 / 1266 / 1224 / 1195 for 0..3 of 4)
   if (L.exp_emu < 0) {
     if (a->dtype != CFK_E4M3) L.exp_emu = a->head_dim == 256 ? 0 : 1;
-    else L.exp_emu = (a->head_dim == 128 && L.variant == 0 && p.sched == 1) ? 1 : 2;
+    else L.exp_emu = (a->head_dim == 128 && (L.variant == 0 || L.variant == 4) && p.sched == 1) ? 1 : 2;
   }
   {
     // Causal: CTAs differ in length, so heads are interleaved (heaviest blocks of a group of heads first);

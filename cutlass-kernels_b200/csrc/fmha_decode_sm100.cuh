@@ -95,7 +95,7 @@ __device__ __forceinline__ uint32_t tile_piece(int row, int even, int bit) {
 template <int DT, int PT, int HD>
 __global__ void __launch_bounds__(160, (DecodeCfg<DT, PT, HD>::CTAS))
 fmha_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const FmhaDecodeParams dp) {
+                   const __grid_constant__ CUtensorMap tm_v, const FmhaSplitParams dp) {
   using C = DecodeCfg<DT, PT, HD>;
   constexpr bool BF16 = PT == kDtBF16;
   const FmhaParams& p = dp.p;

@@ -11,6 +11,13 @@ int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L) {
     if (dtype == CFK_BF16) return fmha_launch_decode_bf16(L, head_dim);
     return p_dtype == CFK_FP16 ? fmha_launch_decode_e4m3_f16(L, head_dim) : fmha_launch_decode_e4m3(L, head_dim);
   }
+  if (L.variant == 4) {
+    const bool d64 = head_dim == 64;
+    if (dtype == CFK_FP16) return d64 ? fmha_launch_tile_f16_f16_64(L) : fmha_launch_tile_f16_f16_128(L);
+    if (dtype == CFK_BF16) return d64 ? fmha_launch_tile_bf16_bf16_64(L) : fmha_launch_tile_bf16_bf16_128(L);
+    if (p_dtype == CFK_FP16) return d64 ? fmha_launch_tile_e4m3_f16_64(L) : fmha_launch_tile_e4m3_f16_128(L);
+    return d64 ? fmha_launch_tile_e4m3_e4m3_64(L) : fmha_launch_tile_e4m3_e4m3_128(L);
+  }
   if (head_dim == 256) {
     if (dtype == CFK_FP16 && p_dtype == CFK_FP16) return fmha_launch_hd256_f16(L);
     if (dtype == CFK_BF16 && p_dtype == CFK_BF16) return fmha_launch_hd256_bf16(L);

@@ -1,0 +1,6 @@
+// One-tile-per-CTA FMHA forward instantiation: Q and K bf16, V and P bf16, head dimension 64.
+#include "fmha_launch_tile_impl.cuh"
+
+namespace cfk {
+int fmha_launch_tile_bf16_bf16_64(const FmhaLaunch& L) { return fmha_launch_tile_t<kDtBF16, kDtBF16, 64>(L); }
+}  // namespace cfk

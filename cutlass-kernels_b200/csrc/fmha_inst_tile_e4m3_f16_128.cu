@@ -1,0 +1,6 @@
+// One-tile-per-CTA FMHA forward instantiation: Q and K e4m3, V and P f16, head dimension 128.
+#include "fmha_launch_tile_impl.cuh"
+
+namespace cfk {
+int fmha_launch_tile_e4m3_f16_128(const FmhaLaunch& L) { return fmha_launch_tile_t<kDtE4M3, kDtF16, 128>(L); }
+}  // namespace cfk

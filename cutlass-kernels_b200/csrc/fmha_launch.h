@@ -14,10 +14,11 @@ struct FmhaLaunch {
   CUtensorMap tm_q, tm_k, tm_v, tm_o;
   CUtensorMap tm_k_half, tm_v_half;   // CTA-pair kernel: boxes of 64 keys x all columns / 128 keys x one 64-column span
   int variant;                        // 0 one CTA per 256 query rows, 1 CTA pairs, 2 persistent, one tile per CTA (see cfk_b200.h),
-                                      // 3 a few query rows against a long cache (fmha_decode_sm100.cuh); never set by the caller
+                                      // 3 a few query rows against a long cache (fmha_decode_sm100.cuh), 4 one 128-row
+                                      // tile per CTA, two CTAs per SM (fmha_fwd_tile_sm100.cuh); these two by size only
   int grid_ctas;                      // variant 2: CTAs of the persistent grid (0 = one per SM)
   FmhaParams p;
-  FmhaDecodeParams dec;               // variant 3: the part of it that is not `p`
+  FmhaSplitParams sp;                 // variants 3 and 4: the part of it that is not `p`
   int iterations;
   int exp_emu;   // 0..3: share (in quarters) of the exponentials computed on the FMA pipe
   cudaStream_t stream;
@@ -52,6 +53,16 @@ int fmha_launch_decode_f16(const FmhaLaunch&, int head_dim);
 int fmha_launch_decode_bf16(const FmhaLaunch&, int head_dim);
 int fmha_launch_decode_e4m3(const FmhaLaunch&, int head_dim);
 int fmha_launch_decode_e4m3_f16(const FmhaLaunch&, int head_dim);
+
+// variant 4: p.nqblk counts 128-row blocks
+int fmha_launch_tile_f16_f16_64(const FmhaLaunch&);
+int fmha_launch_tile_f16_f16_128(const FmhaLaunch&);
+int fmha_launch_tile_bf16_bf16_64(const FmhaLaunch&);
+int fmha_launch_tile_bf16_bf16_128(const FmhaLaunch&);
+int fmha_launch_tile_e4m3_f16_64(const FmhaLaunch&);
+int fmha_launch_tile_e4m3_f16_128(const FmhaLaunch&);
+int fmha_launch_tile_e4m3_e4m3_64(const FmhaLaunch&);
+int fmha_launch_tile_e4m3_e4m3_128(const FmhaLaunch&);
 
 int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L);
 

@@ -19,7 +19,7 @@ int decode_launch(const FmhaLaunch& L) {
       return CFK_ERR_LAUNCH;
     attr_set_for_device = dev;
   }
-  FmhaDecodeParams dp = L.dec;
+  FmhaSplitParams dp = L.sp;
   dp.p = L.p;
   const int ntiles = (L.p.Skv + C::TN - 1) / C::TN;
   const long long ctas = (long long)dp.splits * dp.nqb * L.p.H * L.p.B;

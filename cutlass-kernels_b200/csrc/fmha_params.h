@@ -31,19 +31,21 @@ struct FmhaParams {
   int* status;       // device status word
 };
 
-// The kernel for a few query rows (fmha_decode_sm100.cuh)
+// Keys per tile of the few-rows kernel
 constexpr int decode_tile_keys(int head_dim, int v_bytes) { return head_dim * v_bytes >= 256 ? 64 : 128; }
 // CTAs that share an SM: by shared memory (a tile of K and V of 64 KB), by registers (the output takes head_dim / 2)
 constexpr int decode_ctas_per_sm(int head_dim, int k_bytes, int v_bytes) {
   return decode_tile_keys(head_dim, v_bytes) * head_dim * (k_bytes + v_bytes) >= 65536 ? 1 : (head_dim == 256 ? 2 : 3);
 }
-struct FmhaDecodeParams {
+// The kernels whose clusters share the keys of one block of query rows: a few rows (fmha_decode_sm100.cuh), one 128-row tile
+// (fmha_fwd_tile_sm100.cuh).
+struct FmhaSplitParams {
   FmhaParams p;
   void* o;
   int64_t o_b, o_s, o_h;   // element strides of O
-  int nqb;                 // groups of 16 query rows
-  int nslot;               // slots of the ring of K and V tiles
-  int splits;              // CTAs (a cluster) that share the keys of one (batch, head, group of rows)
+  int nqb;                 // few rows: groups of 16 query rows
+  int nslot;               // few rows: slots of the ring of K and V tiles
+  int splits;              // CTAs (a cluster) that share the keys of one (batch, head, block of rows)
 };
 
 }  // namespace cfk

@@ -171,8 +171,8 @@ const char* cfk_last_cuda_error(void);
  *   CFK_TUNE_FMHA_GROUP_MB  causal only: heads are scheduled in groups whose K and V total at most
  *                           this many MiB (so they share L2), heaviest query blocks first.
  *   CFK_TUNE_FMHA_KERNEL    which FMHA kernel runs: 0 one CTA per 256 query rows (two 128-row tiles side by side), except that
- *                           few query rows (up to 32, or up to 128 with few heads and a long cache) run in a kernel
- *                           that splits the keys over a cluster, so that how a call is cut into heads can change the
+ *                           few query rows, and calls with too few blocks for the SMs, run in kernels of their own,
+ *                           which may split the keys over a cluster: how a call is cut into heads can then change the
  *                           last bit there;
  *                           1 pairs of CTAs (two SMs per 256 rows, tcgen05 cta_group::2; 16-bit inputs with head
  *                           dimension 128 only, other shapes run kernel 0); 2 a persistent grid whose CTAs take one

@@ -1,0 +1,76 @@
+"""Calls with too few 256-row blocks for the SMs run in a kernel with one 128-row tile per CTA.  With whole keys it does the
+same arithmetic in the same order as the 256-row kernel (an explicit schedule selects that one), so the bits are equal; with
+the keys split over a cluster it is compared with the oracle.  Sizes: edges of the 128-row and 128-key tiles, parts without a
+visible key, ragged ends.  Tolerances are those of test_fmha_gpu.py."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import make_qkv, run_fmha
+from test_fmha_gpu import check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,D", [(0, 64), (0, 128), (1, 64), (1, 128), (2, 64), (2, 128)])
+@pytest.mark.parametrize("B,H,Sq,Skv", [(150, 2, 128, 128), (60, 5, 130, 257), (20, 15, 300, 300), (25, 4, 640, 640),
+                                        (75, 4, 33, 385)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_whole_keys_equal_the_256_row_kernel_bit_for_bit(lib, cuda, dtype, D, B, H, Sq, Skv, causal):
+    from cfk_b200 import TUNE_FMHA_SCHED
+    low, _, scales = make_qkv(dtype, B, Sq, Skv, H, D, seed=B)
+    got, stats = run_fmha(lib, low, scales, dtype, causal)
+    try:
+        lib.set_tunable(TUNE_FMHA_SCHED, 1 if dtype == 2 else 0)        # the defaults of the types
+        want, wstats = run_fmha(lib, low, scales, dtype, causal)
+    finally:
+        lib.set_tunable(TUNE_FMHA_SCHED, -1)
+    assert np.array_equal(got, want)
+    for name in stats:
+        assert np.array_equal(stats[name], wstats[name]), name
+
+
+# parts of the keys per tile: 8, 8 (parts of one or two tiles), 4, 2, 8
+@pytest.mark.parametrize("B,H,Sq,Skv", [(1, 4, 256, 2048), (1, 1, 777, 2100), (2, 4, 1024, 1024), (1, 8, 2048, 2048),
+                                        (1, 2, 129, 1921)])
+@pytest.mark.parametrize("dtype,D", [(0, 64), (0, 128), (1, 64), (1, 128), (2, 64), (2, 128)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_split_keys_match_the_oracle(lib, cuda, oracle, dtype, D, B, H, Sq, Skv, causal):
+    low, f32, scales = make_qkv(dtype, B, Sq, Skv, H, D, seed=Skv)
+    got, stats = run_fmha(lib, low, scales, dtype, causal)
+    check(oracle, got, stats, f32, 1.0 / math.sqrt(D), causal, dtype)
+
+
+def test_split_keys_with_low_scores_in_most_parts(lib, cuda, oracle):
+    """Rows whose visible keys lie in the first part only, and scores hundreds of units apart between the parts: the weights
+    of the other parts underflow to zero and must not reach the result."""
+    low, _, scales = make_qkv(0, 1, 1024, 1024, 2, 128, seed=4)
+    q, k, v = low
+    k[0, 512:] *= 0.01
+    k[0, :128] = q[0, :128] * 12
+    f32 = [x.float().numpy() for x in (q, k, v)]
+    for causal in (False, True):
+        got, stats = run_fmha(lib, (q, k, v), scales, 0, causal)
+        check(oracle, got, stats, f32, 1.0 / math.sqrt(128), causal, 0, max_abs=4e-3)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_hybrid_and_a_head_range_split(lib, cuda, oracle, D):
+    """e4m3 Q and K with fp16 V, heads 1 and 2 of five, keys split: strides of the whole tensor; the rest of O stays."""
+    B, H, HT, Sq, Skv = 1, 2, 5, 200, 1500
+    (q, k, _), (qf, kf, _), (qs, ks, _) = make_qkv(2, B, Sq, Skv, HT, D, seed=77)
+    v = torch.randn(B, Skv, HT, D, generator=torch.Generator().manual_seed(78)).half()
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    o = torch.full((B, Sq, HT, D), -7.0, dtype=torch.float16, device="cuda")
+    at = [t.data_ptr() + D * t.element_size() for t in (qd, kd, vd, o)]
+    sq, skv = (Sq * HT * D, HT * D, D), (Skv * HT * D, HT * D, D)
+    lib.fmha_forward(*at, dtype=2, batch=B, heads=H, seqlen_q=Sq, seqlen_kv=Skv, head_dim=D, softmax_scale=D ** -0.5,
+                     causal=True, q_descale=qs, k_descale=ks, v_fp16=True, q_stride=sq, k_stride=skv, v_stride=skv,
+                     o_stride=sq)
+    lib.check_device()
+    cut = lambda x: np.ascontiguousarray(x[:, :, 1:3])    # noqa: E731
+    check(oracle, cut(o.float().cpu().numpy()), {}, (cut(qf), cut(kf), cut(v.float().numpy())), D ** -0.5, True, 0)
+    o[:, :, 1:3] = -7.0
+    assert bool((o == -7.0).all())
