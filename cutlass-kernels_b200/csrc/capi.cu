@@ -275,22 +275,43 @@ static float estimate_us(const cfk_fmha_args* a, int rows, int slots, const Tile
   const float t = sum * (float)bh / (float)slots + c.tail * (c.fixed + c.per_tile * (float)tiles_of(0));
   return (t > longest ? t : longest) + c.offset;
 }
-static int tile_plan(const cfk_fmha_args* a) {
+
+// A remainder of up to 32 rows behind the last whole block takes a CTA per head, as long as any other; without a causal mask it
+// can cost a wave of its own.  It then runs in the few-rows kernel, as a second launch (about 4 us, and the cache once per 16
+// rows at 1.4 times the copy rate), where the estimate says that the wave it saves is worth clearly more.  us, one launch /
+// two: bf16 d = 128, 12 heads, 3080 x 3080: 83.4 / 55.6, 48 heads, 777 x 1300: 44.0 / 40.2, 75 heads, 258 x 1600: 46.7 / 39.1.
+// Below 1024 keys the second launch eats the gain (100 heads, 257 x 400: 25.3 / 26.2), and causal calls, whose CTAs differ in
+// length anyway, lost (48 heads, 777 x 1300: 43.0 / 46.1).
+struct TilePlan { int splits, tail_rows; };   // splits 0: the 256-row kernel
+static TilePlan tile_plan(const cfk_fmha_args* a) {
   constexpr int kSMs = 148;
-  const long long units = (long long)a->batch * a->heads * ((a->seqlen_q + 127) / 128);
+  const long long bh = (long long)a->batch * a->heads, units = bh * ((a->seqlen_q + 127) / 128);
   const int nall = (a->seqlen_kv + 127) / 128;
   if (nall >= 8 && 2 * units <= 2 * kSMs) {
     int s = 2;
     while (s < 8 && units * 2 * s <= 2 * kSMs && nall >= 4 * s) s *= 2;
-    if (s > 2 || nall >= 16) return s;
+    if (s > 2 || nall >= 16) return TilePlan{s, 0};
   }
-  if (nall > 12 || units > 0x7fffffffLL) return 0;
+  if (units > 0x7fffffffLL / 4) return TilePlan{0, 0};
   static const TileCost block256[2][2] = {{{4.31f, 1.33f, 0.86f, 1.45f}, {6.33f, 1.50f, 0.88f, 1.11f}},
                                           {{3.04f, 1.38f, 0.83f, 1.13f}, {4.17f, 1.37f, 0.76f, 0.64f}}};
   static const TileCost tile128[2][2] = {{{4.60f, 1.20f, 1.09f, 1.91f}, {7.11f, 1.49f, 0.99f, 1.33f}},
                                          {{3.33f, 1.20f, 0.83f, 1.86f}, {4.40f, 1.25f, 0.71f, 1.66f}}};   // [e4m3][d = 128]
   const int e = a->dtype == CFK_E4M3 && !a->v_fp16, d = a->head_dim == 128;
-  return estimate_us(a, 128, 2 * kSMs, tile128[e][d]) < 0.94f * estimate_us(a, 256, kSMs, block256[e][d]) ? 1 : 0;
+  TilePlan plan{0, 0};
+  if (nall <= 12 && estimate_us(a, 128, 2 * kSMs, tile128[e][d]) < 0.94f * estimate_us(a, 256, kSMs, block256[e][d]))
+    plan.splits = 1;
+  const int rows = plan.splits ? 128 : 256, slots = plan.splits ? 2 * kSMs : kSMs, rest = a->seqlen_q % rows;
+  const long long blocks = bh * (a->seqlen_q / rows);        // whole ones
+  if (!a->causal && nall >= 8 && rest > 0 && rest <= 32 && a->seqlen_q > rows) {
+    const long long waves = (blocks + slots - 1) / slots, waves_all = (blocks + bh + slots - 1) / slots;
+    const TileCost& c = plan.splits ? tile128[e][d] : block256[e][d];
+    const float wave = c.fixed + c.per_tile * (float)nall;
+    const float bytes = (float)bh * (float)((rest + 15) / 16) * (float)a->seqlen_kv * (float)a->head_dim *
+                        (float)(dtype_size(a->dtype) + (a->v_fp16 ? 2 : dtype_size(a->dtype)));
+    if ((float)waves * wave + 4.f + 1.4f * bytes / 6.65e6f < 0.85f * (float)waves_all * wave) plan.tail_rows = rest;
+  }
+  return plan;
 }
 
 // Argument checks, TMA descriptors, kernel parameters and kernel choice of one FMHA call: everything of the launch
@@ -337,8 +358,8 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   const bool by_size = L.variant == 0 && sched < 0 && !a->s_dump;
   const bool decode = by_size && decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim);
   if (decode) L.variant = 3;
-  const int tile_splits = by_size && !decode && a->head_dim != 256 ? tile_plan(a) : 0;
-  if (tile_splits > 0) L.variant = 4;
+  const TilePlan plan = by_size && !decode && a->head_dim != 256 ? tile_plan(a) : TilePlan{0, 0};
+  if (plan.splits > 0) L.variant = 4;
   const int q_rows = decode ? 16 : 128, kv_rows = decode ? decode_tile_keys(a->head_dim, dtype_size(vdt)) : 128;
   if ((rc = encode_bshd(&L.tm_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], q_rows)))
     return rc;
@@ -352,11 +373,27 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
     return rc;
   L.sp.o = a->o;
   L.sp.o_b = os[0]; L.sp.o_s = os[1]; L.sp.o_h = os[2];
-  L.sp.splits = tile_splits;
+  L.sp.splits = plan.splits;
   if (decode) {
     L.sp.nqb = (a->seqlen_q + 15) / 16;
     L.sp.splits = decode_splits(groups16, (a->seqlen_kv + kv_rows - 1) / kv_rows,
                                  148 * decode_ctas_per_sm(a->head_dim, esz, dtype_size(vdt)));
+  }
+
+  if (plan.tail_rows > 0) {   // the last rows run in the few-rows kernel
+    const int keys = decode_tile_keys(a->head_dim, dtype_size(vdt));
+    if ((rc = encode_bshd(&L.tail_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], 16)))
+      return rc;
+    if ((rc = encode_bshd(&L.tail_k, a->dtype, a->k, a->batch, a->seqlen_kv, a->heads, a->head_dim, ks[0], ks[1], ks[2], keys)))
+      return rc;
+    if ((rc = encode_bshd(&L.tail_v, vdt, a->v, a->batch, a->seqlen_kv, a->heads, a->head_dim, vs[0], vs[1], vs[2], keys)))
+      return rc;
+    L.tail_rows = plan.tail_rows;
+    L.tail_sp = L.sp;
+    L.tail_sp.nqb = (plan.tail_rows + 15) / 16;
+    L.tail_sp.row_first = a->seqlen_q - plan.tail_rows;
+    L.tail_sp.splits = decode_splits((long long)a->batch * a->heads * L.tail_sp.nqb, (a->seqlen_kv + keys - 1) / keys,
+                                     148 * decode_ctas_per_sm(a->head_dim, esz, dtype_size(vdt)));
   }
 
   L.grid_ctas = g_tunable[CFK_TUNE_FMHA_GRID].load();
@@ -373,6 +410,7 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   p.out_bf16 = a->out_dtype == CFK_BF16;
   // one 128-row tile per CTA at head dimension 256 and in kernels 2 and 4, two side by side otherwise
   p.nqblk = (a->head_dim == 256 || L.variant == 2 || L.variant == 4) ? (a->seqlen_q + 127) / 128 : (a->seqlen_q + 255) / 256;
+  if (L.tail_rows > 0) p.nqblk -= 1;
   {
     // Default by input type, the measured best: with e4m3 Q and K the first GEMM is short enough for the two query
     // tiles to take turns on one score buffer (+8-12 % on every e4m3 shape together with the share of exponentials on

@@ -117,7 +117,7 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const int rank = (int)blockIdx.x % dp.splits, unit = (int)blockIdx.x / dp.splits;
   const int qb = unit % dp.nqb, bh = unit / dp.nqb;
   const int batch = bh / p.H, head = bh - batch * p.H;
-  const int row0 = qb * C::ROWS;
+  const int row0 = dp.row_first + qb * C::ROWS;
   const int nrows = min(C::ROWS, p.Sq - row0);
   const int diag_off = p.Skv - p.Sq;
   const int visible = p.causal ? min(p.Skv, row0 + nrows + diag_off) : p.Skv;   // keys the last row sees

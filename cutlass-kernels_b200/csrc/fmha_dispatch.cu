@@ -5,7 +5,7 @@
 
 namespace cfk {
 
-int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L) {
+static int dispatch_one(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L) {
   if (L.variant == 3) {
     if (dtype == CFK_FP16) return fmha_launch_decode_f16(L, head_dim);
     if (dtype == CFK_BF16) return fmha_launch_decode_bf16(L, head_dim);
@@ -46,6 +46,16 @@ int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L) {
   if (dtype == CFK_E4M3 && p_dtype == CFK_E4M3)
     return head_dim == 64 ? fmha_launch_e4m3_e4m3_64(L) : head_dim == 128 ? fmha_launch_e4m3_e4m3_128(L) : CFK_ERR_UNSUPPORTED;
   return CFK_ERR_UNSUPPORTED;
+}
+
+int fmha_dispatch(int dtype, int p_dtype, int head_dim, const FmhaLaunch& L) {
+  const int rc = dispatch_one(dtype, p_dtype, head_dim, L);
+  if (rc != CFK_OK || L.tail_rows == 0) return rc;
+  FmhaLaunch tail = L;
+  tail.variant = 3;
+  tail.tm_q = L.tail_q; tail.tm_k = L.tail_k; tail.tm_v = L.tail_v;
+  tail.sp = L.tail_sp;
+  return dispatch_one(dtype, p_dtype, head_dim, tail);
 }
 
 }  // namespace cfk

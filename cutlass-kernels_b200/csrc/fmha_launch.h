@@ -19,6 +19,9 @@ struct FmhaLaunch {
   int grid_ctas;                      // variant 2: CTAs of the persistent grid (0 = one per SM)
   FmhaParams p;
   FmhaSplitParams sp;                 // variants 3 and 4: the part of it that is not `p`
+  int tail_rows;                      // last rows of the call that run in the few-rows kernel, after the launch above (0: none)
+  CUtensorMap tail_q, tail_k, tail_v;
+  FmhaSplitParams tail_sp;
   int iterations;
   int exp_emu;   // 0..3: share (in quarters) of the exponentials computed on the FMA pipe
   cudaStream_t stream;

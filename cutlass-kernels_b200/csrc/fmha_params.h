@@ -44,6 +44,7 @@ struct FmhaSplitParams {
   void* o;
   int64_t o_b, o_s, o_h;   // element strides of O
   int nqb;                 // few rows: groups of 16 query rows
+  int row_first;           // few rows: the first of them (0, or behind the rows another launch does)
   int nslot;               // few rows: slots of the ring of K and V tiles
   int splits;              // CTAs (a cluster) that share the keys of one (batch, head, block of rows)
 };
