@@ -324,7 +324,10 @@ fmha_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                          "r"(oreg[4 * g]), "r"(oreg[4 * g + 1]), "r"(oreg[4 * g + 2]), "r"(oreg[4 * g + 3]) : "memory");
         }
       }
-      const bool none = n_kv == 0 || l == 0.f;
+      // No visible key, or none with a score above -inf.  The sum does not tell: masked keys add 2^-126 each where the
+      // exponential is taken on the FMA pipe, against a reference maximum of 0.  A sum of NaN (NaN scores, which a maximum
+      // passes over) is passed on.
+      const bool none = n_kv == 0 || (m_true == -INFINITY && l == l);
       asm volatile("st.shared.f32 [%0], %1;" ::"r"(sStat + tid * 4), "f"(none ? -INFINITY : mref2) : "memory");
       asm volatile("st.shared.f32 [%0], %1;" ::"r"(sStat + 512 + tid * 4), "f"(none ? 0.f : l) : "memory");
       asm volatile("st.shared.f32 [%0], %1;" ::"r"(sStat + 1024 + tid * 4), "f"(m_true * sl) : "memory");

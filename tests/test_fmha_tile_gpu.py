@@ -56,6 +56,42 @@ def test_split_keys_with_low_scores_in_most_parts(lib, cuda, oracle):
         check(oracle, got, stats, f32, 1.0 / math.sqrt(128), causal, 0, max_abs=4e-3)
 
 
+def very_negative(dtype, Sq, Skv, H, D, seed):
+    """make_qkv with every scaled score near -120: Q around +c, K around -c in every element, c^2 sqrt(D) = 120."""
+    low, _, _ = make_qkv(0, 1, Sq, Skv, H, D, seed=seed)
+    c = math.sqrt(120 / math.sqrt(D))
+    q, k, v = low[0].float() * 0.3 + c, low[1].float() * 0.3 - c, low[2].float()
+    if dtype == 2:
+        scales = [float(x.abs().max()) / 448.0 for x in (q, k, v)]
+        low = [(x / s).to(torch.float8_e4m3fn) for x, s in zip((q, k, v), scales)]
+    else:
+        scales = [1.0, 1.0, 1.0]
+        low = [x.to((torch.float16, torch.bfloat16)[dtype]) for x in (q, k, v)]
+    return low, [(x.float() * s).numpy() for x, s in zip(low, scales)], scales
+
+
+# Four parts, and a diagonal that falls into the middle of a key tile: the last tiles of a block are invisible to its first
+# rows, so that a part has key tiles but no visible key for a row (84 and 204 pairs of row and part per head).
+@pytest.mark.parametrize("Sq,Skv", [(1000, 1100), (900, 960)])
+@pytest.mark.parametrize("dtype,D", [(0, 64), (0, 128), (1, 64), (1, 128), (2, 64), (2, 128)])
+def test_parts_with_keys_but_none_visible_to_a_row_have_no_weight(lib, cuda, oracle, dtype, D, Sq, Skv):
+    """Against maxima far below zero: such a part must not pass for one whose largest score is zero."""
+    low, f32, scales = very_negative(dtype, Sq, Skv, 4, D, seed=Sq)
+    got, stats = run_fmha(lib, low, scales, dtype, True)
+    check(oracle, got, stats, f32, 1.0 / math.sqrt(D), True, dtype)
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_a_part_whose_scores_are_all_minus_infinity_has_no_weight(lib, cuda, oracle, dtype):
+    """Keys 512 to 1023 (two of eight parts) at -inf against positive Q: as if they were not there, V included."""
+    low, f32, scales = very_negative(dtype, 512, 2048, 4, 128, seed=3)
+    low[1][:, 512:1024] = -math.inf
+    got, stats = run_fmha(lib, low, scales, dtype, False)
+    keep = np.r_[0:512, 1024:2048]
+    check(oracle, got, stats, [f32[0], np.ascontiguousarray(f32[1][:, keep]), np.ascontiguousarray(f32[2][:, keep])],
+          1.0 / math.sqrt(128), False, dtype)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_hybrid_and_a_head_range_split(lib, cuda, oracle, D):
     """e4m3 Q and K with fp16 V, heads 1 and 2 of five, keys split: strides of the whole tensor; the rest of O stays."""
