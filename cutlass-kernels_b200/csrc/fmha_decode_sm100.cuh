@@ -209,7 +209,10 @@ fmha_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const int lim1 = p.causal ? min(p.Skv - 1, row0 + (lane >> 2) + 8 + diag_off) : p.Skv - 1;
     const int min_lim = p.causal ? min(p.Skv - 1, row0 + diag_off) : p.Skv - 1;
     bool split = false;
-    if constexpr (BF16) split = (p.causal ? min(p.Skv, row0 + diag_off + 1) : p.Skv) < p.split_keys;
+    if constexpr (BF16) {   // by the first row of the 256-row block (d = 256: 128), as in the kernels that take such blocks
+      const int first = row0 & ~(HD == 256 ? 127 : 255);
+      split = (p.causal ? min(p.Skv, first + diag_off + 1) : p.Skv) < p.split_keys;
+    }
     const int k16 = warp * C::NK;                                // this warp's keys within a tile
     const int kb_row = k16 + (lane & 7) + (C::ESZ == 2 ? ((lane >> 4) & 1) : ((lane >> 3) & 1)) * 8;
     const int kb_chunk = C::ESZ == 2 ? (lane >> 3) & 1 : lane >> 4;

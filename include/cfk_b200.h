@@ -56,9 +56,8 @@ typedef struct cfk_fmha_args {
   int out_dtype;  /* cfk_dtype of O: FP16 or BF16 */
   int p_split_keys; /* P (unnormalised probabilities) is rounded to the input type before P*V, as the
                        reference does (fmha_consumer.h:54).  bf16 only: query blocks (256 rows; 128 at head
-                       dimension 256; 16 where few rows meet a long cache) whose first row sees fewer keys than
-                       this keep P as a two-term bf16 sum (hi + lo, two MMAs), because
-                       with few keys bf16's 8-bit rounding of P is not averaged out.
+                       dimension 256) whose first row sees fewer keys than this keep P as a two-term bf16 sum
+                       (hi + lo, two MMAs), because with few keys bf16's 8-bit rounding of P is not averaged out.
                        -1 = default (1024), 0 = never.  Ignored for fp16 / e4m3. */
   int batch, heads, seqlen_q, seqlen_kv, head_dim;
   const void* q;

@@ -27,6 +27,20 @@ def test_few_rows_match_the_oracle(lib, cuda, oracle, D, dtype, causal):
         check(oracle, got, stats, f32, 1.0 / math.sqrt(D), causal, dtype)
 
 
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("Sq,Skv", [(30, 1040), (100, 1100)])
+def test_bf16_rows_keep_the_two_term_p_of_their_whole_block(lib, cuda, oracle, D, Sq, Skv):
+    """The first row sees fewer than 1024 keys, so P is a sum of two bf16 terms for every row of the call, as in the kernels with
+    blocks of 256 (d = 256: 128) rows, also where a group of 16 rows begins above 1024.  The rounding of O to fp16 is then
+    what is left, 2^-12 at most and about 2.0e-4 in the mean of squares; one bf16 term of P gives 1.5e-3."""
+    low, f32, scales = make_qkv(1, 1, Sq, Skv, 2, D, seed=Sq)
+    got, _ = run_fmha(lib, low, scales, 1, True)
+    want = oracle.attention(f32[0], f32[1], f32[2], 1.0 / math.sqrt(D), True)["o"]
+    for row in range(0, Sq, 16):
+        d, w = (got - want)[:, row:row + 16], want[:, row:row + 16]
+        assert np.sqrt((d ** 2).sum() / (w ** 2).sum()) < 5e-4, row
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_few_rows_hybrid_and_a_head_range_of_a_wider_tensor(lib, cuda, oracle, D):
     """e4m3 Q and K with fp16 V (the hybrid mode), heads 1 and 2 of five: strides of the whole tensor, and the other heads
