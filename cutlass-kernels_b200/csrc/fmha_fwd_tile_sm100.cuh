@@ -340,8 +340,11 @@ fmha_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           w[c] = c < sp.splits ? ld_shared_cluster_f32(map_to_cta(sStat + tid * 4, c)) : -INFINITY;
           mx = fmaxf(mx, w[c]);
         }
+        // Parts that have left an O.  Those whose weight underflows to 0 count: NaN and infinite values reach the result.
+        uint32_t has = 0u;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
+          if (w[c] != -INFINITY) has |= 1u << c;
           w[c] = w[c] == -INFINITY ? 0.f : ex2_approx(w[c] - mx);
           if (c < sp.splits) {
             lsum += w[c] * ld_shared_cluster_f32(map_to_cta(sStat + 512 + tid * 4, c));
@@ -355,7 +358,7 @@ fmha_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            if (w[c] != 0.f) {                                 // a part without a visible key has left no O
+            if (has >> c & 1u) {                               // a part without a visible key has left no O
               const float4 v = ld_shared_cluster_f32x4(map_to_cta(sRing + g * 2048 + tid * 16, c));
               acc.x += w[c] * v.x; acc.y += w[c] * v.y; acc.z += w[c] * v.z; acc.w += w[c] * v.w;
             }

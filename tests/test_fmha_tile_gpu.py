@@ -92,6 +92,39 @@ def test_a_part_whose_scores_are_all_minus_infinity_has_no_weight(lib, cuda, ora
           1.0 / math.sqrt(128), False, dtype)
 
 
+@pytest.mark.parametrize("what", ["value of a key without weight", "value", "key", "query", "score"])
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("dtype,Sq", [(0, 256), (1, 256), (0, 20), (1, 20)])
+def test_nan_and_infinity_reach_the_outputs_they_reach_with_whole_keys(lib, cuda, dtype, Sq, bad, what):
+    """Split keys (256 rows: eight parts of one tile; 20 rows: the few-rows kernel) against the 256-row kernel, which takes all
+    keys of a row in order: the same elements of O and lse are finite.  Keys from 512 on score about -120, so that their
+    probability is zero next to the others'."""
+    from cfk_b200 import TUNE_FMHA_SCHED
+    low, _, scales = very_negative(dtype, Sq, 2048, 2, 128, seed=1)
+    q, k, v = low
+    k[:, :512] = make_qkv(dtype, 1, Sq, 512, 2, 128, seed=2)[0][1] * 0.1
+    if what == "value of a key without weight":
+        v[0, 1000, 1, 5] = bad
+    elif what == "value":
+        v[0, 100, 1, 5] = bad
+    elif what == "key":
+        k[0, 1100, 0] = bad
+    elif what == "query":
+        q[0, 17, 1] = bad
+    else:                                  # one score of +inf (NaN after the maximum is taken away)
+        k[0, 1500, 0] = math.inf if bad == math.inf else 0
+        k[0, 1500, 0, 0] = bad
+    got, stats = run_fmha(lib, low, scales, dtype, False)
+    try:
+        lib.set_tunable(TUNE_FMHA_SCHED, 0)
+        want, wstats = run_fmha(lib, low, scales, dtype, False)
+    finally:
+        lib.set_tunable(TUNE_FMHA_SCHED, -1)
+    assert not np.isfinite(want).all()
+    assert np.array_equal(np.isfinite(got), np.isfinite(want))
+    assert np.array_equal(np.isfinite(stats["lse"]), np.isfinite(wstats["lse"]))
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_hybrid_and_a_head_range_split(lib, cuda, oracle, D):
     """e4m3 Q and K with fp16 V, heads 1 and 2 of five, keys split: strides of the whole tensor; the rest of O stays."""
