@@ -379,11 +379,17 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Another CTA's shared memory, and tensor memory allocated for a pair, may be touched only once that CTA is known to have
+// started: every thread of the cluster arrives at the top of the kernel and waits ahead of the first such access.  In
+// between a CTA sets up what is its own, so the wait is for the slowest start and nothing else.
+__device__ __forceinline__ void cluster_arrive_started() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_started() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The skip decision of a cluster (see cta_should_skip), taken ONCE for all its CTAs: if each CTA read the status word
 // for itself, another CTA's wait could give up between two reads, one CTA of a pair would return and its peer
 // would go on to allocate tensor memory for the pair (which has no time limit) and to signal barriers in the shared
 // memory of a CTA that is gone.  Rank 0 reads the word and stores the decision into every CTA's shared memory; after
-// the cluster barrier each branches on its own copy.  Every thread of every CTA must call this.
+// the cluster barrier each branches on its own copy.  Every thread of every CTA must call this, and all CTAs of the
+// cluster must be known to have started (cluster_wait_started).
 __device__ __forceinline__ bool cluster_should_skip(const int* status, int ctas) {
   __shared__ uint32_t s_cluster_skip;
   if (threadIdx.x == 0 && cluster_ctarank() == 0) {

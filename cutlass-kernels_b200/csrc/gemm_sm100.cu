@@ -167,6 +167,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   const int nks_all = (p.K + bk * C::KSUB - 1) / (bk * C::KSUB);
   const int ks0 = nks_all * part / p.splits, nks = nks_all * (part + 1) / p.splits - ks0;   // this pair's stages of k-blocks
 
+  cluster_arrive_started();
   grid_dependency_launch();
   if (tid == 0) {
     for (int i = 0; i < C::NSTAGE; ++i) { mbar_init(bar_full + 8 * i, 2); mbar_init(bar_empty + 8 * i, 1); }
@@ -175,6 +176,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
     *s_abort = 0u;
     fence_barrier_init();
   }
+  __syncwarp();
+  cluster_wait_started();
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(s_tmem_base)), 2 * TN);
     tmem_relinquish_pair();

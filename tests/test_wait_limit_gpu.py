@@ -35,3 +35,40 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_library_usable(lib, ora
     got, _ = run_fmha(lib, low, scales, 0, False, want_stats=False)
     ref = oracle.attention(f32[0], f32[1], f32[2], 1.0 / math.sqrt(128), False)["o"]
     assert np.abs(got - ref).max() <= 2e-3
+
+
+@pytest.mark.parametrize("what", ["gemm pairs", "gemm clusters of 8", "attention pairs", "few rows", "split keys", "remainder"])
+def test_clusters_skip_together_behind_a_wait_that_ran_out(lib, cuda, what):
+    """One decision per cluster, taken by one CTA: with the status word set nothing is written and every CTA leaves; once it is
+    clear the same call runs."""
+    from cfk_b200 import TUNE_FMHA_KERNEL
+    g = torch.Generator().manual_seed(5)
+
+    def gemm(m, n, k):
+        a, b = (torch.randn(r, k, generator=g).half().cuda() for r in (m, n))
+        c = torch.full((n, m), -1.0, device="cuda", dtype=torch.float16)
+        return c, lambda: lib.gemm(a, b, c, dtype=0, m=m, n=n, k=k)
+
+    def fmha(H, Sq, Skv):
+        low, _, _ = make_qkv(0, 1, Sq, Skv, H, 128, seed=Sq)
+        q, k, v = (x.cuda() for x in low)
+        o = torch.full((1, Sq, H, 128), -1.0, device="cuda", dtype=torch.float16)
+        return o, lambda: lib.fmha_forward(q, k, v, o, dtype=0, batch=1, heads=H, seqlen_q=Sq, seqlen_kv=Skv, head_dim=128,
+                                           softmax_scale=128 ** -0.5)
+
+    out, call = {"gemm pairs": lambda: gemm(4096, 5120, 64), "gemm clusters of 8": lambda: gemm(8, 8, 2056),
+                 "attention pairs": lambda: fmha(2, 300, 300), "few rows": lambda: fmha(2, 4, 4000),
+                 "split keys": lambda: fmha(2, 256, 2048), "remainder": lambda: fmha(12, 3080, 3080)}[what]()
+    lib.check_device()
+    try:
+        if what == "attention pairs":
+            lib.set_tunable(TUNE_FMHA_KERNEL, 1)
+        assert lib.selftest_wait_gives_up(20) == 0
+        call()
+        assert lib.device_status() == (6, 901)
+        assert bool((out == -1.0).all())
+        call()
+        lib.check_device()
+        assert bool((out != -1.0).float().mean() > 0.99)
+    finally:
+        lib.set_tunable(TUNE_FMHA_KERNEL, -1)
