@@ -122,8 +122,10 @@ __device__ __forceinline__ void settle_if_aborted(volatile uint32_t* cta_abort) 
 // launch before may have written (inputs, status word) is read, and nothing is written, ahead of the wait; every thread
 // executes it, so a launch never completes before its predecessor.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The launch after this one may start filling SMs once every CTA of this launch has executed this (or left): from then
-// on no CTA of this launch is still waiting for an SM.
+// The launch after this one may start filling SMs once a thread of every CTA of this launch has executed this (or the CTA
+// has left): from then on no CTA of this launch is still waiting for an SM.  Kernels with tensor memory execute it in the
+// warp that allocates, after the allocation: tcgen05.alloc waits without a limit, and a CTA of the next launch that had
+// taken the columns first would in turn wait for this launch to end.
 __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // CTA-uniform test of the status word (one thread reads, everybody gets the same answer).

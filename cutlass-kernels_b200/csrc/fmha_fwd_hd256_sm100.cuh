@@ -109,7 +109,6 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
 
   // Set-up as in fmha_fwd_sm100.cuh: ahead of the wait for the launch before, with Q and K_0 on their way early.
-  grid_dependency_launch();
   if (warp == 5 && lane == 0) {
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < C::NSLOT; ++i) {
@@ -139,6 +138,7 @@ fmha_fwd_hd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (warp == 4) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(s_tmem_base)), C::TMEM_COLS);
     tmem_relinquish();
+    grid_dependency_launch();
   }
   if (warp == 5) __syncwarp();
   grid_dependency_wait();

@@ -103,7 +103,6 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // ---- set-up ----
   // Everything up to grid_dependency_wait() overlaps the launch before this one.  The producer thread sets the barriers
   // up itself, so that Q and K_0 are on their way before the CTA meets at the __syncthreads.
-  grid_dependency_launch();
   if (warp == 9 && lane == 0) {
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < C::NSLOT; ++i) {
@@ -134,6 +133,7 @@ fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == 8) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(s_tmem_base)), C::TMEM_COLS);
     tmem_relinquish();
+    grid_dependency_launch();
   }
   if (warp == 9) __syncwarp();
   grid_dependency_wait();

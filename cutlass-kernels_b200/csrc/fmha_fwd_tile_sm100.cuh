@@ -94,7 +94,6 @@ fmha_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int n_kv = n_all * (part + 1) / sp.splits - j0;
 
   // Set-up as in fmha_fwd_sm100.cuh: ahead of the wait for the launch before, with Q and the first K on their way early.
-  grid_dependency_launch();
   if (warp == 5 && lane == 0) {
     mbar_init(bar_q_full, 1);
     for (int i = 0; i < C::NSLOT; ++i) { mbar_init(bar_kv_full + 8 * i, 1); mbar_init(bar_kv_empty + 8 * i, 1); }
@@ -120,6 +119,7 @@ fmha_fwd_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (warp == 4) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(s_tmem_base)), C::TMEM_COLS);
     tmem_relinquish();
+    grid_dependency_launch();
   }
   if (warp == 5) __syncwarp();
   grid_dependency_wait();

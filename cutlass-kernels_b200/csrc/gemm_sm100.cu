@@ -168,7 +168,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   const int ks0 = nks_all * part / p.splits, nks = nks_all * (part + 1) / p.splits - ks0;   // this pair's stages of k-blocks
 
   cluster_arrive_started();
-  grid_dependency_launch();
   if (tid == 0) {
     for (int i = 0; i < C::NSTAGE; ++i) { mbar_init(bar_full + 8 * i, 2); mbar_init(bar_empty + 8 * i, 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(bar_acc_full + 8 * i, 1); mbar_init(bar_acc_empty + 8 * i, 256); }
@@ -181,6 +180,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(s_tmem_base)), 2 * TN);
     tmem_relinquish_pair();
+    grid_dependency_launch();
   }
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tm_x); tma_prefetch_desc(&tm_y); tma_prefetch_desc(&tm_d); }
   grid_dependency_wait();

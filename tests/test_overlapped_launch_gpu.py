@@ -41,3 +41,37 @@ def test_chained_calls_equal_the_chain_with_waits(lib, cuda, D, S, side_stream):
 
     for a, b in zip(chain(False), chain(True)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,D", [(0, 64), (2, 64), (1, 128)])
+def test_kernels_with_tensor_memory_follow_each_other_on_an_sm(lib, cuda, dtype, D):
+    """Launches of half an SM (one-tile attention), of a whole one (256-row attention, d = 256) and of CTA pairs (GEMM), each on
+    its way while the one before it runs: the results are those of the launches with waits between them."""
+    g = torch.Generator().manual_seed(D)
+    cast = {0: torch.float16, 1: torch.bfloat16, 2: torch.float8_e4m3fn}
+    at = {}
+    for name, (B, S, hd) in {"one tile": (300, 128, D), "block": (2, 400, D), "d256": (2, 300, 256)}.items():
+        q, k, v = (torch.randn(B, S, 1, hd, generator=g).to(cast[dtype]).cuda() for _ in range(3))
+        at[name] = (B, S, hd, q, k, v)
+    a, b = (torch.randn(r, 512, generator=g).half().cuda() for r in (768, 1024))
+
+    def chain(wait):
+        outs = []
+        for i in range(4):
+            for name, (B, S, hd, q, k, v) in at.items():
+                o = torch.zeros(B, S, 1, hd, dtype=torch.float16, device="cuda")
+                lib.fmha_forward(q, k, v, o, dtype=dtype, batch=B, heads=1, seqlen_q=S, seqlen_kv=S, head_dim=hd,
+                                 softmax_scale=hd ** -0.5, causal=bool(i & 1))
+                outs.append(o)
+                if wait:
+                    torch.cuda.synchronize()
+                c = torch.zeros(1024, 768, dtype=torch.float16, device="cuda")
+                lib.gemm(a, b, c, dtype=0, m=768, n=1024, k=512)
+                outs.append(c)
+                if wait:
+                    torch.cuda.synchronize()
+        lib.check_device()
+        return outs
+
+    for x, y in zip(chain(False), chain(True)):
+        assert torch.equal(x, y)
