@@ -21,7 +21,7 @@ STATUS_NAMES = {0: "OK", 1: "INVALID_ARG", 2: "UNSUPPORTED", 3: "DESCRIPTOR", 4:
                 6: "DEVICE_WAIT", 7: "TOO_LARGE"}
 
 EXPORTS = ["cfk_fmha_forward", "cfk_fmha_forward_static", "cfk_gemm", "cfk_fill", "cfk_convert", "cfk_device_status",
-           "cfk_last_cuda_error", "cfk_version", "cfk_selftest_umma", "cfk_umma_peak", "cfk_selftest_wait_gives_up", "cfk_selftest_wait_gives_up_static", "cfk_set_tunable", "cfk_get_tunable"]
+           "cfk_last_cuda_error", "cfk_version", "cfk_selftest_umma", "cfk_umma_peak", "cfk_selftest_wait_gives_up", "cfk_selftest_wait_gives_up_static", "cfk_set_tunable", "cfk_get_tunable", "cfk_fmha_plan", "cfk_gemm_plan"]
 
 TUNE_FMHA_EXP_EMU, TUNE_FMHA_GROUP_MB, TUNE_FMHA_KERNEL, TUNE_FMHA_GRID, TUNE_FMHA_SCHED = 0, 1, 2, 3, 4
 
@@ -93,6 +93,8 @@ class CfkLib:
         L.cfk_last_cuda_error.restype = C.c_char_p
         L.cfk_selftest_umma.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p] + [C.c_int] * 5 + [C.c_void_p]
         L.cfk_umma_peak.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_double), C.c_void_p]
+        L.cfk_fmha_plan.argtypes = [C.POINTER(FmhaArgs), C.POINTER(C.c_int)]
+        L.cfk_gemm_plan.argtypes = [C.POINTER(GemmArgs), C.POINTER(C.c_int)]
         L.cfk_selftest_wait_gives_up.argtypes = [C.c_int, C.c_void_p]
         L.cfk_selftest_wait_gives_up_static.argtypes = [C.c_int, C.c_void_p]
 
@@ -141,6 +143,22 @@ class CfkLib:
                                         1 if c_row_major else 0, iterations, _ptr(c_src)), stream)
         if rc:
             raise CfkError(rc, self.last_error())
+
+    def fmha_plan(self, args: FmhaArgs):
+        """(kernel, key parts, remainder rows, key parts of the remainder) of a call; launches nothing, needs no device."""
+        plan = (C.c_int * 4)()
+        rc = int(self.lib.cfk_fmha_plan(C.byref(args), plan))
+        if rc:
+            raise CfkError(rc, self.last_error())
+        return tuple(plan)
+
+    def gemm_plan(self, args: GemmArgs):
+        """(tile width, parts of the reduction, operands exchanged) of a call on the current device; launches nothing."""
+        plan = (C.c_int * 3)()
+        rc = int(self.lib.cfk_gemm_plan(C.byref(args), plan))
+        if rc:
+            raise CfkError(rc, self.last_error())
+        return tuple(plan)
 
     def fill(self, dst, dtype, n, seed, kind="normal", scale=1.0, value=0.0, first_index=0, stream=None) -> None:
         kinds = {"normal": 0, "uniform": 1, "const": 2, "integers": 3}

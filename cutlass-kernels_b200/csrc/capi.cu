@@ -314,10 +314,10 @@ static TilePlan tile_plan(const cfk_fmha_args* a) {
   return plan;
 }
 
-// Argument checks, TMA descriptors, kernel parameters and kernel choice of one FMHA call: everything of the launch
-// except the status pointer and the stream, which the two entry points supply (allocated block / static array).
-// *p_dtype receives the type P is rounded to (and V is stored in).
-int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
+static int v_dtype(const cfk_fmha_args* a) { return a->v_fp16 ? CFK_FP16 : a->dtype; }   // V, and what P is rounded to
+static float descale(const cfk_fmha_args* a, float x) { return a->dtype != CFK_E4M3 && x == 0.f ? 1.f : x; }
+
+static int check_fmha_args(const cfk_fmha_args* a) {
   if (!a || !a->q || !a->k || !a->v || !a->o) return CFK_ERR_INVALID_ARG;
   if (a->batch <= 0 || a->heads <= 0 || a->seqlen_q <= 0 || a->seqlen_kv <= 0 || a->iterations < 0)
     return CFK_ERR_INVALID_ARG;
@@ -329,12 +329,58 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   if (a->causal && a->seqlen_kv < a->seqlen_q) return CFK_ERR_UNSUPPORTED;
   if (a->p_split_keys < -1) return CFK_ERR_INVALID_ARG;
   if (a->v_fp16 && (a->dtype != CFK_E4M3 || a->head_dim == 256)) return CFK_ERR_UNSUPPORTED;
-  const int vdt = a->v_fp16 ? CFK_FP16 : a->dtype;   // element type of V, and the type P is rounded to
-  const int pdt = vdt;
-  const float qd = a->dtype == CFK_E4M3 ? a->q_descale : (a->q_descale == 0.f ? 1.f : a->q_descale);
-  const float kd = a->dtype == CFK_E4M3 ? a->k_descale : (a->k_descale == 0.f ? 1.f : a->k_descale);
-  const float vd = a->dtype == CFK_E4M3 ? a->v_descale : (a->v_descale == 0.f ? 1.f : a->v_descale);
-  if (!(qd > 0.f) || !(kd > 0.f) || !(vd > 0.f)) return CFK_ERR_INVALID_ARG;
+  if (!(descale(a, a->q_descale) > 0.f) || !(descale(a, a->k_descale) > 0.f) || !(descale(a, a->v_descale) > 0.f))
+    return CFK_ERR_INVALID_ARG;
+  return CFK_OK;
+}
+
+// Which kernel a call runs, from its sizes, types and the knobs alone.
+struct FmhaChoice {
+  int variant;                    // FmhaLaunch::variant
+  int splits;                     // variants 3 and 4: CTAs that share a block's keys
+  int tail_rows, tail_splits;     // last rows of the call that run in the few-rows kernel, and its splits
+  int sched;                      // the knob; negative: by type
+};
+static int few_rows_splits(const cfk_fmha_args* a, int rows) {
+  const int esz = dtype_size(a->dtype), vsz = dtype_size(v_dtype(a)), keys = decode_tile_keys(a->head_dim, vsz);
+  return decode_splits((long long)a->batch * a->heads * ((rows + 15) / 16), (a->seqlen_kv + keys - 1) / keys,
+                       148 * decode_ctas_per_sm(a->head_dim, esz, vsz));
+}
+static FmhaChoice choose_kernel(const cfk_fmha_args* a) {
+  tunables_from_env();
+  FmhaChoice c = {g_tunable[CFK_TUNE_FMHA_KERNEL].load(), 0, 0, 0, g_tunable[CFK_TUNE_FMHA_SCHED].load()};
+  if (c.variant == 1 && (a->dtype == CFK_E4M3 || a->head_dim != 128)) c.variant = 0;
+  if (a->head_dim == 256) c.variant = 0;
+  if (c.variant != 0 || c.sched >= 0 || a->s_dump) return c;   // an explicit schedule asks for the kernel that has one
+  const long long groups16 = (long long)a->batch * a->heads * ((a->seqlen_q + 15) / 16);
+  if (decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim)) {
+    c.variant = 3;
+    c.splits = few_rows_splits(a, a->seqlen_q);
+  } else if (a->head_dim != 256) {
+    const TilePlan plan = tile_plan(a);
+    if (plan.splits > 0) c.variant = 4;
+    c.splits = plan.splits;
+    c.tail_rows = plan.tail_rows;
+    if (c.tail_rows > 0) c.tail_splits = few_rows_splits(a, c.tail_rows);
+  }
+  return c;
+}
+
+extern "C" int cfk_fmha_plan(const cfk_fmha_args* a, int plan[4]) {
+  const int rc = check_fmha_args(a);
+  if (rc != CFK_OK || !plan) return rc != CFK_OK ? rc : CFK_ERR_INVALID_ARG;
+  const FmhaChoice c = choose_kernel(a);
+  plan[0] = c.variant; plan[1] = c.splits; plan[2] = c.tail_rows; plan[3] = c.tail_splits;
+  return CFK_OK;
+}
+
+// Argument checks, TMA descriptors, kernel parameters and kernel choice of one FMHA call: everything of the launch
+// except the status pointer and the stream, which the two entry points supply (allocated block / static array).
+// *p_dtype receives the type P is rounded to (and V is stored in).
+int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
+  int rc = check_fmha_args(a);
+  if (rc != CFK_OK) return rc;
+  const int vdt = v_dtype(a);
   const uintptr_t align_or = (uintptr_t)a->q | (uintptr_t)a->k | (uintptr_t)a->v | (uintptr_t)a->o;
   if (align_or & 15u) return CFK_ERR_INVALID_ARG;
 
@@ -345,21 +391,11 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
   if (!resolve_strides(a->v_stride, vs, a->seqlen_kv, a->heads, a->head_dim, dtype_size(vdt))) return CFK_ERR_INVALID_ARG;
   if (!resolve_strides(a->o_stride, os, a->seqlen_q, a->heads, a->head_dim, 2)) return CFK_ERR_INVALID_ARG;
 
-  tunables_from_env();
   FmhaLaunch& L = *out;
   std::memset(&L, 0, sizeof(L));
-  int rc;
-  L.variant = g_tunable[CFK_TUNE_FMHA_KERNEL].load();
-  if (L.variant == 1 && (a->dtype == CFK_E4M3 || a->head_dim != 128)) L.variant = 0;
-  if (a->head_dim == 256) L.variant = 0;
-  const long long groups16 = (long long)a->batch * a->heads * ((a->seqlen_q + 15) / 16);
-  // an explicit schedule asks for the kernel that has one
-  const int sched = g_tunable[CFK_TUNE_FMHA_SCHED].load();
-  const bool by_size = L.variant == 0 && sched < 0 && !a->s_dump;
-  const bool decode = by_size && decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim);
-  if (decode) L.variant = 3;
-  const TilePlan plan = by_size && !decode && a->head_dim != 256 ? tile_plan(a) : TilePlan{0, 0};
-  if (plan.splits > 0) L.variant = 4;
+  const FmhaChoice choice = choose_kernel(a);
+  L.variant = choice.variant;
+  const bool decode = L.variant == 3;
   const int q_rows = decode ? 16 : 128, kv_rows = decode ? decode_tile_keys(a->head_dim, dtype_size(vdt)) : 128;
   if ((rc = encode_bshd(&L.tm_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], q_rows)))
     return rc;
@@ -373,14 +409,10 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
     return rc;
   L.sp.o = a->o;
   L.sp.o_b = os[0]; L.sp.o_s = os[1]; L.sp.o_h = os[2];
-  L.sp.splits = plan.splits;
-  if (decode) {
-    L.sp.nqb = (a->seqlen_q + 15) / 16;
-    L.sp.splits = decode_splits(groups16, (a->seqlen_kv + kv_rows - 1) / kv_rows,
-                                 148 * decode_ctas_per_sm(a->head_dim, esz, dtype_size(vdt)));
-  }
+  L.sp.splits = choice.splits;
+  L.sp.nqb = (a->seqlen_q + 15) / 16;
 
-  if (plan.tail_rows > 0) {   // the last rows run in the few-rows kernel
+  if (choice.tail_rows > 0) {   // the last rows run in the few-rows kernel
     const int keys = decode_tile_keys(a->head_dim, dtype_size(vdt));
     if ((rc = encode_bshd(&L.tail_q, a->dtype, a->q, a->batch, a->seqlen_q, a->heads, a->head_dim, qs[0], qs[1], qs[2], 16)))
       return rc;
@@ -388,12 +420,11 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
       return rc;
     if ((rc = encode_bshd(&L.tail_v, vdt, a->v, a->batch, a->seqlen_kv, a->heads, a->head_dim, vs[0], vs[1], vs[2], keys)))
       return rc;
-    L.tail_rows = plan.tail_rows;
+    L.tail_rows = choice.tail_rows;
     L.tail_sp = L.sp;
-    L.tail_sp.nqb = (plan.tail_rows + 15) / 16;
-    L.tail_sp.row_first = a->seqlen_q - plan.tail_rows;
-    L.tail_sp.splits = decode_splits((long long)a->batch * a->heads * L.tail_sp.nqb, (a->seqlen_kv + keys - 1) / keys,
-                                     148 * decode_ctas_per_sm(a->head_dim, esz, dtype_size(vdt)));
+    L.tail_sp.nqb = (choice.tail_rows + 15) / 16;
+    L.tail_sp.row_first = a->seqlen_q - choice.tail_rows;
+    L.tail_sp.splits = choice.tail_splits;
   }
 
   L.grid_ctas = g_tunable[CFK_TUNE_FMHA_GRID].load();
@@ -416,11 +447,11 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
     // tiles to take turns on one score buffer (+8-12 % on every e4m3 shape together with the share of exponentials on
     // the FMA pipe that goes with it, below); with 16-bit inputs the hand-over of
     // the buffer would set the pace (c3 1246 -> 1221 TFLOP/s).
-    p.sched = sched < 0 ? (a->dtype == CFK_E4M3 ? 1 : 0) : sched;
+    p.sched = choice.sched < 0 ? (a->dtype == CFK_E4M3 ? 1 : 0) : choice.sched;
   }
   p.split_keys = a->dtype == CFK_BF16 ? (a->p_split_keys < 0 ? 1024 : a->p_split_keys) : 0;
-  p.scale_log2 = a->softmax_scale * 1.4426950408889634f * qd * kd;
-  p.out_scale = vd;
+  p.scale_log2 = a->softmax_scale * 1.4426950408889634f * descale(a, a->q_descale) * descale(a, a->k_descale);
+  p.out_scale = descale(a, a->v_descale);
   p.lse = a->lse; p.mi = a->mi; p.sprime = a->sprime;
   p.s_dump = a->s_dump; p.s_dump_bf16 = a->dtype == CFK_BF16;
   L.iterations = a->iterations;
@@ -440,7 +471,7 @@ int cfk::fmha_prepare(const cfk_fmha_args* a, FmhaLaunch* out, int* p_dtype) {
     p.group = (int)(grp < 1 ? 1 : (grp > bh ? bh : grp));
   }
   if ((long long)p.nqblk * a->heads * a->batch > 0x7fffffffLL) return CFK_ERR_UNSUPPORTED;
-  *p_dtype = pdt;
+  *p_dtype = vdt;
   return CFK_OK;
 }
 

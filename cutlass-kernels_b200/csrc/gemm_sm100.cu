@@ -567,12 +567,27 @@ static int launch_gemm(const CUtensorMap& tm_x, const CUtensorMap& tm_y, const C
 
 using namespace cfk;
 
-extern "C" int cfk_gemm(const cfk_gemm_args* a, cfk_stream_t stream) {
+static int check_gemm_args(const cfk_gemm_args* a) {
   if (!a || !a->a || !a->b || !a->c) return CFK_ERR_INVALID_ARG;
   if (a->m <= 0 || a->n <= 0 || a->k <= 0 || a->l <= 0 || a->iterations < 0) return CFK_ERR_INVALID_ARG;
   if (a->dtype != CFK_FP16 && a->dtype != CFK_BF16 && a->dtype != CFK_FP32) return CFK_ERR_UNSUPPORTED;
   if ((a->m % 8) || (a->n % 8) || (a->k % 8)) return CFK_ERR_UNSUPPORTED;
   if (((uintptr_t)a->a | (uintptr_t)a->b | (uintptr_t)a->c | (uintptr_t)a->c_src) & 15u) return CFK_ERR_INVALID_ARG;
+  return CFK_OK;
+}
+
+extern "C" int cfk_gemm_plan(const cfk_gemm_args* a, int plan[3]) {
+  const int rc = check_gemm_args(a);
+  if (rc != CFK_OK || !plan) return rc != CFK_OK ? rc : CFK_ERR_INVALID_ARG;
+  const GemmPlan g = a->c_row_major ? plan_gemm(a->m, a->n, a->k, a->l, a->dtype == CFK_FP32)
+                                    : plan_gemm(a->n, a->m, a->k, a->l, a->dtype == CFK_FP32);
+  plan[0] = g.tn; plan[1] = g.splits; plan[2] = g.trans;
+  return CFK_OK;
+}
+
+extern "C" int cfk_gemm(const cfk_gemm_args* a, cfk_stream_t stream) {
+  int rc = check_gemm_args(a);
+  if (rc != CFK_OK) return rc;
 
   int err = CFK_OK;
   int* status = device_status_block(&err);
@@ -590,7 +605,6 @@ extern "C" int cfk_gemm(const cfk_gemm_args* a, cfk_stream_t stream) {
   CUtensorMap tm_x, tm_y, tm_d;
   const uint64_t esz = (uint64_t)dtype_size(a->dtype);
   const uint32_t bk = (uint32_t)(128 / esz);                   // one 128-byte span of the reduction per stage
-  int rc;
   auto operand = [&](CUtensorMap* tm, const void* base, int rows, int box_rows) {
     const uint64_t d[3] = {(uint64_t)a->k, (uint64_t)rows, (uint64_t)a->l};
     const uint64_t st[2] = {(uint64_t)a->k * esz, (uint64_t)a->k * esz * (uint64_t)rows};

@@ -138,6 +138,19 @@ typedef struct cfk_gemm_args {
 int cfk_gemm(const cfk_gemm_args* args, cfk_stream_t stream);
 
 /*
+ * Which kernel a call would run, for tests and profiles; launches nothing.  No counterpart in the reference, which chooses
+ * at compile time.  The choice depends on sizes, types and the knobs below, never on addresses or contents.
+ * cfk_fmha_plan (needs no device): plan[0] = 0, 1, 2 the kernels of CFK_TUNE_FMHA_KERNEL (0 at head dimension 256: the
+ * kernel for that size), 3 the one for few query rows, 4 the one with a single 128-row tile per CTA; plan[1] = CTAs that
+ * share the keys of a block of rows in kernels 3 and 4 (1: whole keys), else 0; plan[2] = last query rows that run in
+ * kernel 3 in a launch of their own (0: none), plan[3] = CTAs that share the keys there.
+ * cfk_gemm_plan (asks the current device how many clusters it holds): plan[0] = tile width, plan[1] = CTA pairs that share
+ * the reduction of a tile, plan[2] = 1 if the operands are exchanged.
+ */
+int cfk_fmha_plan(const cfk_fmha_args* args, int plan[4]);
+int cfk_gemm_plan(const cfk_gemm_args* args, int plan[3]);
+
+/*
  * Device-side random fills, element i depends only on (seed, first_index + i).
  * Replaces cfk::initialize_rand / initialize_const (include/utils/random.hpp:20-50).
  * kind 0: N(0,1); kind 1: U[-1,1]; kind 2: constant `value`.  The result is value * scale

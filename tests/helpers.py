@@ -41,3 +41,18 @@ def run_fmha(lib, low, scales, dtype, causal, out_dtype=0, p_split_keys=-1, want
                      lse=stats.get("lse"), mi=stats.get("mi"), sprime=stats.get("sprime"))
     lib.check_device()
     return o.float().cpu().numpy(), {k2: v2.cpu().numpy() for k2, v2 in stats.items()}
+
+
+BLOCK, FEW_ROWS, ONE_TILE = 0, 3, 4     # kernels of fmha_plan
+
+
+def fmha_plan(lib, dtype, B, H, Sq, Skv, D, causal, v_fp16=False, **kw):
+    """Which kernel such a call runs: (kernel, key parts, remainder rows, key parts of the remainder)."""
+    return lib.fmha_plan(lib.fmha_args(0x1000, 0x2000, 0x3000, 0x4000, dtype=dtype, batch=B, heads=H, seqlen_q=Sq,
+                                       seqlen_kv=Skv, head_dim=D, softmax_scale=D ** -0.5, causal=causal, v_fp16=v_fp16, **kw))
+
+
+def gemm_plan(lib, M, N, K, L, row_major, dtype):
+    """(tile width, parts of the reduction, operands exchanged) of such a call on this device."""
+    import cfk_b200
+    return lib.gemm_plan(cfk_b200.GemmArgs(dtype, M, N, K, L, 0x1000, 0x2000, 0x3000, 1.0, 0.0, int(row_major), 1, None))

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import make_qkv, run_fmha
+from helpers import BLOCK, fmha_plan, make_qkv, run_fmha
 from test_fmha_gpu import check
 
 pytestmark = pytest.mark.gpu
@@ -100,3 +100,20 @@ def test_fmha_schedules_agree_bit_for_bit(lib, cuda, dtype, causal):
     assert np.array_equal(outs[0][0], outs[1][0])
     for name in outs[0][1]:
         assert np.array_equal(outs[0][1][name], outs[1][1][name]), name
+
+
+@pytest.mark.parametrize("dtype", [0, 1, 2])
+@pytest.mark.parametrize("Sq,Skv", [(300, 2100), (1024, 1024)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_many_key_tiles_at_head_dimension_64_match_the_oracle(lib, oracle, cuda, dtype, Sq, Skv, causal):
+    """The 256-row kernel going round its ring of K and V tiles at head dimension 64.  By size such a small call would run in the
+    kernel that splits the keys; an explicit schedule (there is only one at this head dimension) keeps it here."""
+    from cfk_b200 import TUNE_FMHA_SCHED
+    low, f32, scales = make_qkv(dtype, 1, Sq, Skv, 2, 64, seed=Sq + dtype)
+    lib.set_tunable(TUNE_FMHA_SCHED, 0)
+    try:
+        assert fmha_plan(lib, dtype, 1, 2, Sq, Skv, 64, causal) == (BLOCK, 0, 0, 0)
+        got, stats = run_fmha(lib, low, scales, dtype, causal)
+    finally:
+        lib.set_tunable(TUNE_FMHA_SCHED, -1)
+    check(oracle, got, stats, f32, 1.0 / math.sqrt(64), causal, dtype)

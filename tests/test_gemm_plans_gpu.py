@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+from helpers import gemm_plan
 from test_gemm_gpu import run
 
 pytestmark = pytest.mark.gpu
@@ -19,7 +20,10 @@ SHAPES = [(8, 8, 8, 1, False),            # 64
           (8, 8, 1032, 1, False),         # 64 / 3: column units without an owner
           (8, 1544, 1032, 3, True),       # 64 / 3, exchanged
           (8, 8, 2056, 1, False),         # 64 / 4
-          (8, 2056, 1032, 1, True),       # 64 / 4, exchanged
+          (8, 2056, 1032, 1, True),       # 64 / 2
+          (8, 776, 1032, 3, True),        # 64 / 4, exchanged
+          (72, 3080, 4104, 3, True),      # 128, exchanged
+          (72, 1544, 1032, 3, True),      # 128 / 3, exchanged
           (16, 1544, 72, 3, True),        # 128
           (136, 776, 2056, 3, False),     # 128 / 2
           (72, 2056, 2056, 3, True),      # 128 / 2, exchanged
@@ -29,6 +33,15 @@ SHAPES = [(8, 8, 8, 1, False),            # 64
           (264, 776, 2056, 3, True),      # 256 / 2
           (264, 2056, 2056, 1, True),     # 256 / 3
           (1032, 520, 4104, 1, False)]    # 256 / 4
+# tile width, pairs that share a tile's reduction, operands exchanged
+PLANS = [(64, 1, 0), (64, 1, 1), (64, 2, 0), (64, 2, 1), (64, 3, 0), (64, 3, 1), (64, 4, 0), (64, 2, 0), (64, 4, 1),
+         (128, 1, 1), (128, 3, 1), (128, 1, 0), (128, 2, 0), (128, 2, 1), (128, 3, 0), (128, 4, 0), (128, 4, 1),
+         (256, 2, 0), (256, 3, 0), (256, 4, 0)]
+
+
+def test_the_shapes_reach_the_plans(lib, cuda):
+    assert [gemm_plan(lib, *s, dtype=1) for s in SHAPES] == PLANS
+    assert gemm_plan(lib, 8192, 8192, 8192, 1, False, dtype=0) == (256, 1, 0)
 
 
 @pytest.mark.parametrize("M,N,K,L,row_major", SHAPES)

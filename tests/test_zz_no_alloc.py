@@ -97,3 +97,16 @@ def test_static_entry_point_reports_a_wait_that_gave_up_and_the_next_call_clears
     assert lib.fmha_forward_static_raw(_args(lib, low, got, scales, 0, True)) == 0
     assert lib.fmha_forward_static_raw(_args(lib, low, got, scales, 0, True, iterations=0)) == 0
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("H,Sq,Skv,causal", [(3, 5, 700, True), (300, 128, 128, True), (4, 256, 2048, False), (12, 3080, 3080, False)])
+def test_static_entry_point_takes_the_same_route_by_size(lib, cuda, H, Sq, Skv, causal):
+    """The kernels for few rows, for one tile (whole keys, split keys) and the second launch for a remainder of rows."""
+    low, _, scales = make_qkv(0, 1, Sq, Skv, H, 128, seed=Sq)
+    low = [x.cuda() for x in low]
+    want, got = (torch.full((1, Sq, H, 128), x, device="cuda", dtype=torch.float16) for x in (-1.0, -2.0))
+    assert lib.fmha_forward_raw(_args(lib, low, want, scales, 0, causal)) == 0
+    lib.check_device()
+    assert lib.fmha_forward_static_raw(_args(lib, low, got, scales, 0, causal)) == 0
+    assert lib.fmha_forward_static_raw(_args(lib, low, got, scales, 0, causal, iterations=0)) == 0
+    assert torch.equal(got, want)
