@@ -231,12 +231,26 @@ static bool resolve_strides(const int64_t in[3], int64_t out[3], int S, int H, i
 //   128 x 1628: 22.0 / 11.4; beyond that it loses: 64 heads, 64 x 1564: 24.1 / 23.5, 200 heads, 64 x 364: 22.4 / 27.3; short
 //   caches of so many rows are launch-bound either way;
 //   d = 256, where the other kernel already has one 128-row tile per CTA and a tile here fills an SM: four CTAs or more per
-//   group, 24 heads, 8 x 6008: 62.6 / 29.6; with fewer it is even: 64 heads, 16 x 1516: 23.4 / 25.2.
-static bool decode_is_faster(long long groups, int sq, int skv, int head_dim) {
+//   group, 24 heads, 8 x 6008: 62.6 / 29.6; with fewer it is even: 64 heads, 16 x 1516: 23.4 / 25.2;
+//   17 to 32 rows, two groups per head, d = 128 and 16-bit V: not where the groups run over what is resident at once (444) into
+//   as many waves as the 256-row kernel has of its one CTA per head, that is with 223 to 296 heads: 256 heads, 32 x 2048:
+//   54 / 66, 32 x 8192: 212 / 257; 222 and 297 heads 53 / 44 and 76 / 70.  Not so with the two-term P of bf16, which costs the
+//   256-row kernel more (256 heads, 32 x 800: 38 / 36), and with e4m3 V (256 heads, 32 x 4096: 84 / 79).
+static bool decode_is_faster(const cfk_fmha_args* a) {
   constexpr int kSMs = 148;
+  const int sq = a->seqlen_q, skv = a->seqlen_kv;
+  const long long bh = (long long)a->batch * a->heads, groups = bh * ((sq + 15) / 16);
   if (groups > 0x7fffffffLL / 8) return false;
-  if (head_dim == 256) return sq <= 128 && skv >= 1024 && 4 * groups <= kSMs;
-  return sq <= 32 || (sq <= 128 && skv >= 1024 && groups <= kSMs);
+  if (a->head_dim == 256) return sq <= 128 && skv >= 1024 && 4 * groups <= kSMs;
+  if (sq > 32) return sq <= 128 && skv >= 1024 && groups <= kSMs;
+  const bool v16 = a->dtype != CFK_E4M3 || a->v_fp16;
+  const int first = a->causal ? skv - sq + 1 : skv;            // keys the first row sees
+  const bool two_term = a->dtype == CFK_BF16 && first < (a->p_split_keys < 0 ? 1024 : a->p_split_keys);
+  if (sq > 16 && a->head_dim == 128 && v16 && !two_term && bh > kSMs) {
+    const int resident = kSMs * decode_ctas_per_sm(128, dtype_size(a->dtype), 2);
+    return (groups + resident - 1) / resident < (bh + kSMs - 1) / kSMs;
+  }
+  return true;
 }
 
 // CTAs (a cluster) per group of 16 rows: as many as are resident at once, with two tiles of keys each at least; 8 is the
@@ -352,8 +366,7 @@ static FmhaChoice choose_kernel(const cfk_fmha_args* a) {
   if (c.variant == 1 && (a->dtype == CFK_E4M3 || a->head_dim != 128)) c.variant = 0;
   if (a->head_dim == 256) c.variant = 0;
   if (c.variant != 0 || c.sched >= 0 || a->s_dump) return c;   // an explicit schedule asks for the kernel that has one
-  const long long groups16 = (long long)a->batch * a->heads * ((a->seqlen_q + 15) / 16);
-  if (decode_is_faster(groups16, a->seqlen_q, a->seqlen_kv, a->head_dim)) {
+  if (decode_is_faster(a)) {
     c.variant = 3;
     c.splits = few_rows_splits(a, a->seqlen_q);
   } else if (a->head_dim != 256) {

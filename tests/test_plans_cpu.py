@@ -22,6 +22,13 @@ from helpers import BLOCK, FEW_ROWS, ONE_TILE, fmha_plan
     (0, 1, 37, 16, 1024, 256, False, (FEW_ROWS, 4, 0, 0)),       # d = 256: four CTAs or more per group
     (0, 1, 38, 16, 1024, 256, False, (BLOCK, 0, 0, 0)),
     (0, 1, 37, 16, 1023, 256, False, (BLOCK, 0, 0, 0)),
+    (0, 2, 111, 32, 4096, 128, False, (FEW_ROWS, 1, 0, 0)),      # two groups per head: one wave of 444 ..
+    (0, 1, 223, 32, 4096, 128, False, (BLOCK, 0, 0, 0)),         # .. two, as the 256-row kernel has ..
+    (1, 4, 74, 17, 4096, 128, True, (BLOCK, 0, 0, 0)),
+    (1, 4, 74, 17, 800, 128, True, (FEW_ROWS, 1, 0, 0)),         # (two-term P)
+    (0, 4, 74, 16, 4096, 128, True, (FEW_ROWS, 1, 0, 0)),        # (one group per head)
+    (2, 4, 74, 32, 4096, 128, False, (FEW_ROWS, 1, 0, 0)),       # (e4m3 V)
+    (0, 1, 297, 32, 4096, 128, False, (FEW_ROWS, 1, 0, 0)),      # .. two against three
     (0, 1, 8, 300, 896, 128, False, (BLOCK, 0, 0, 0)),           # split keys from 8 key tiles on, that is 897 keys
     (0, 1, 8, 300, 897, 128, False, (ONE_TILE, 4, 0, 0)),
     (0, 1, 12, 3080, 3080, 128, False, (BLOCK, 0, 8, 8)),        # a remainder of 8 rows
