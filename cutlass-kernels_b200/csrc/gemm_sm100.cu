@@ -411,22 +411,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CU
           for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
           if (p.trans) {       // the warp's 32 rows are neighbours in D
             const size_t at = (size_t)b * p.d_batch + (size_t)col * p.ldd + row;
-            if (p.beta != 0.f) {                       // all reads ahead of the first write, which might be to the same matrix
-              float old[32];
+            // All reads ahead of the first write, which might be to the same matrix, and ahead of any use: converted one by one
+            // they waited for each other (16-bit, 64 x 3088 x 1032 with beta, 14.8 us).
+            if (p.beta != 0.f) {
+              uint32_t old[32];
 #pragma unroll
               for (int i = 0; i < 32; ++i) {
-                old[i] = 0.f;
+                old[i] = 0u;
                 if (col + i < p.Cn) {
-                  if (p.tf32) {
-                    old[i] = reinterpret_cast<const float*>(p.src)[at + (size_t)i * p.ldd];
-                  } else {
-                    const uint16_t h = reinterpret_cast<const uint16_t*>(p.src)[at + (size_t)i * p.ldd];
-                    old[i] = p.bf16 ? __uint_as_float((uint32_t)h << 16) : __half2float(__ushort_as_half(h));
-                  }
+                  const size_t e = at + (size_t)i * p.ldd;
+                  old[i] = p.tf32 ? reinterpret_cast<const uint32_t*>(p.src)[e] : reinterpret_cast<const uint16_t*>(p.src)[e];
                 }
               }
 #pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] += p.beta * old[i];
+              for (int i = 0; i < 32; ++i)
+                v[i] += p.beta * (p.tf32 ? __uint_as_float(old[i])
+                                         : p.bf16 ? __uint_as_float(old[i] << 16) : __half2float(__ushort_as_half((uint16_t)old[i])));
             }
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
