@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cmath>
 #include <cstring>
 #include <utility>
 
@@ -505,7 +506,10 @@ static const int* resident_clusters() {   // [splits]
 // be faster, 256 without a split.  Below that SMs stand idle, and the estimate decides, in us: a fixed part (launch, first
 // loads, epilogue), a time per k-block of the longest chain of tiles (a narrower tile costs less, but not in proportion; rows
 // whose pitch is not a multiple of 32 bytes make TMA fetch every sector's neighbour too), the exchange of a split, and for
-// exchanged operands, which pay where D has few rows, the two-byte stores of each column a CTA finishes.  The constants are
+// exchanged operands, which pay where D has few rows, the two-byte stores of each column a CTA finishes.  Every further wave
+// of tiles costs its epilogue besides its k-blocks, and with rows of less than 128 bytes the load of many short rows; without
+// that a short reduction went to narrow tiles in many waves: 256 x 18944 x 8 in bf16 14.1 us against 9.8 with one wave of 256,
+// x 64 8.8 / 7.2, fp32 x 520 14.7 / 13.2, fp32 256 x 30000 x 8 23.2 / 13.1.  The constants are
 // fits to a sweep of 24 shapes x 2 orders x 18 plans in bf16 and fp32; the plan it chose was the fastest or within 5 % of it
 // for nearly all.  us before / after, bf16: 2048 x 768 x 4096 25.4 / 16.4, 16 x 3088 x 9968 50.4 / 12.8, 1408 x 536 x 2816
 // 19.3 / 11.2, 88 x 88 x 80 6.9 / 5.2.
@@ -520,6 +524,9 @@ static GemmPlan plan_gemm(int R, int Cn, int K, int L, bool fp32) {
   const bool pitch32 = pitch % 32 == 0;
   static const float fixed[3] = {6.3f, 5.3f, 4.8f};
   static const float per_kb[2][3] = {{0.37f, 0.33f, 0.29f}, {0.30f, 0.17f, 0.15f}};
+  static const float wave_fixed[2][3] = {{2.3f, 1.5f, 1.0f}, {3.7f, 2.0f, 1.2f}};     // [fp32]
+  static const float wave_kb[3] = {0.31f, 0.23f, 0.23f};
+  const float short_rows = pitch < 128 ? 4.f * (1.f - (float)pitch / 128.f) : 0.f;
   static const float exchange[3][5] = {{0, 0, 2.8f, 3.5f, 4.4f}, {0, 0, 1.9f, 2.4f, 3.0f}, {0, 0, 1.4f, 2.1f, 2.4f}};
   float best_t = 0.f;
   for (int trans = 0; trans < 2; ++trans)
@@ -529,7 +536,9 @@ static GemmPlan plan_gemm(int R, int Cn, int K, int L, bool fp32) {
         const long long tiles = trans ? tiles_of(Cn, R, tn) : tiles_of(R, Cn, tn);
         if (s > stages || ((s > 1 || trans) && tiles > resident[s])) continue;
         const long long waves = (tiles + pairs - 1) / pairs;
-        float t = fixed[w] + per_kb[pitch32][w] * (float)((nkb + s - 1) / s) * (float)waves + exchange[w][s];
+        const float kb = (float)((nkb + s - 1) / s);
+        float t = fixed[w] + per_kb[pitch32][w] * kb + exchange[w][s];
+        if (waves > 1) t += (float)(waves - 1) * (fmaxf(wave_fixed[fp32][w], short_rows) + fmaxf(per_kb[pitch32][w], wave_kb[w]) * kb);
         if (trans) t += 0.3f + 0.03f * (float)(R < tn ? R : tn) / (float)s;
         if (best_t == 0.f || t < best_t) { best_t = t; best = GemmPlan{tn, s, trans}; }
       }

@@ -25,6 +25,7 @@ SHAPES = [(8, 8, 8, 1, False),            # 64
           (72, 3080, 4104, 3, True),      # 128, exchanged
           (72, 1544, 1032, 3, True),      # 128 / 3, exchanged
           (16, 1544, 72, 3, True),        # 128
+          (720, 9456, 64, 1, True),       # 128, three waves
           (136, 776, 2056, 3, False),     # 128 / 2
           (72, 2056, 2056, 3, True),      # 128 / 2, exchanged
           (72, 776, 1032, 3, True),       # 128 / 3
@@ -35,13 +36,18 @@ SHAPES = [(8, 8, 8, 1, False),            # 64
           (1032, 520, 4104, 1, False)]    # 256 / 4
 # tile width, pairs that share a tile's reduction, operands exchanged
 PLANS = [(64, 1, 0), (64, 1, 1), (64, 2, 0), (64, 2, 1), (64, 3, 0), (64, 3, 1), (64, 4, 0), (64, 2, 0), (64, 4, 1),
-         (128, 1, 1), (128, 3, 1), (128, 1, 0), (128, 2, 0), (128, 2, 1), (128, 3, 0), (128, 4, 0), (128, 4, 1),
+         (128, 1, 1), (128, 3, 1), (128, 1, 0), (128, 1, 0), (128, 2, 0), (128, 2, 1), (128, 3, 0), (128, 4, 0), (128, 4, 1),
          (256, 2, 0), (256, 3, 0), (256, 4, 0)]
 
 
 def test_the_shapes_reach_the_plans(lib, cuda):
     assert [gemm_plan(lib, *s, dtype=1) for s in SHAPES] == PLANS
     assert gemm_plan(lib, 8192, 8192, 8192, 1, False, dtype=0) == (256, 1, 0)
+    assert gemm_plan(lib, 2048, 768, 4096, 1, False, dtype=0) == (128, 1, 0)
+    # a short reduction does not pay for further waves of narrow tiles
+    for M, N, K, L, dtype in ((256, 18944, 8, 1, 1), (256, 18944, 64, 1, 1), (776, 3992, 136, 1, 1), (256, 30000, 8, 1, 3),
+                              (464, 2040, 520, 4, 3), (1024, 1024, 264, 8, 3)):
+        assert gemm_plan(lib, M, N, K, L, True, dtype) == (256, 1, 0), (M, N, K, L, dtype)
 
 
 @pytest.mark.parametrize("M,N,K,L,row_major", SHAPES)
