@@ -53,15 +53,17 @@ __global__ void __launch_bounds__(256) convert_kernel(const void* src, void* dst
 template <int SDT, int DDT>
 static cudaError_t launch_convert(const void* src, void* dst, int64_t n, float scale, cudaStream_t stream) {
   constexpr int SB = elem_bytes(SDT), DB = elem_bytes(DDT);
-  constexpr int V = 16 / (SB > DB ? SB : DB), U = 2;
+  constexpr int V = 16 / (SB > DB ? SB : DB), U = 2, U1 = 8;
   // Vectors need both addresses to be a multiple of their own width.  Otherwise, and where the whole array is less than
-  // one vector, one element per access.  fp32 -> e4m3 at 67.1 M elements (335 MB): 49.7 us back to back, 6.7 TB/s, against
-  // 116.9 one element at a time.  Alone with a cold L2, by U: 1: 73.7, 2: 55.3, 4: 56.2, 8: 55.3; small sizes are launch-bound.
+  // one vector, one element per access, and more of them in flight per thread.  fp32 -> e4m3 at 67.1 M elements (335 MB): 49.7 us
+  // back to back, 6.7 TB/s, against 116.9 one element at a time in a grid-stride loop.  Alone with a cold L2, by U: 1: 73.7,
+  // 2: 55.3, 4: 56.2, 8: 55.3; small sizes are launch-bound.  Off by one element, by U1: 2: 136, 4: 69.2, 8: 50.1, 16: 57.2;
+  // 9 M elements 19.1 / 10.3 / 7.0 / 7.9 (grid-stride loop: 125 and 11.2).
   const bool vec = n >= V && ((uintptr_t)src % (V * SB)) == 0 && ((uintptr_t)dst % (V * DB)) == 0;
-  const int64_t per_block = 256 * U * (int64_t)(vec ? V : 1);
+  const int64_t per_block = 256 * (int64_t)(vec ? U * V : U1);
   const int64_t blocks = (n + per_block - 1) / per_block;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  auto kern = vec ? convert_kernel<SDT, DDT, V, U> : convert_kernel<SDT, DDT, 1, U>;
+  auto kern = vec ? convert_kernel<SDT, DDT, V, U> : convert_kernel<SDT, DDT, 1, U1>;
   return launch_overlapped(kern, dim3((unsigned)blocks), dim3(256), 0, stream, src, dst, n, scale);
 }
 

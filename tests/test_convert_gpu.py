@@ -14,7 +14,8 @@ BITS = {1: torch.uint8, 2: torch.int16, 4: torch.int32}
 def test_convert_matches_the_casts_bit_for_bit(lib, cuda, src, dst):
     g = torch.Generator().manual_seed(10 * src + dst)
     for n, off_s, off_d in [(1, 0, 0), (3, 0, 0), (15, 0, 0), (16, 0, 0), (17, 0, 0), (2048, 0, 0), (2047 + 8192, 0, 0),
-                            (4099, 1, 0), (4099, 0, 1), (5000, 3, 5), (5000, 16, 16), (300007, 0, 0)]:
+                            (4099, 1, 0), (4099, 0, 1), (5000, 3, 5), (5000, 16, 16), (300007, 0, 0),
+                            (2047, 1, 0), (2048, 0, 1), (2049, 1, 1), (300007, 1, 3)]:
         x = torch.randn(n + off_s, generator=g) * 100
         for i, special in enumerate((0.0, -0.0, float("inf"), float("-inf"), float("nan"), 1e-7, 447.0, 1e6)):
             if n > 20:
