@@ -179,13 +179,21 @@ const char* cfk_last_cuda_error(void);
  * (src/fmha-pipeline/shared_storage.h:3-32).
  *   CFK_TUNE_FMHA_EXP_EMU   0..3: of every four pairs of softmax exponentials, how many are evaluated
  *                           with a cubic on the FMA pipe instead of the special-function unit.  -1 (default):
- *                           by input type and head dimension, the measured best.
+ *                           by input type and head dimension, the measured best.  The kernel for few query rows
+ *                           takes none there, whatever the value.
  *   CFK_TUNE_FMHA_GROUP_MB  causal only: heads are scheduled in groups whose K and V total at most
- *                           this many MiB (so they share L2), heaviest query blocks first.
+ *                           this many MiB (so they share L2), heaviest query blocks first.  No effect in the
+ *                           kernel for few query rows, whose blocks are equally long.
  *   CFK_TUNE_FMHA_KERNEL    which FMHA kernel runs: 0 one CTA per 256 query rows (two 128-row tiles side by side), except that
- *                           few query rows, and calls with too few blocks for the SMs, run in kernels of their own,
- *                           which may split the keys over a cluster: how a call is cut into heads can then change the
- *                           last bit there;
+ *                           few query rows, a short remainder of rows, and calls with too few blocks for the SMs run in
+ *                           kernels of their own, which may split the keys over a cluster (cfk_fmha_plan says which).
+ *                           That choice looks at batch x heads.  So the same head can come out differently in a call
+ *                           of its own, or in a rank's share, than in the whole call, within the accuracy of the type but not
+ *                           in the last bit only: P is rounded against another maximum, and e4m3 inputs keep P in fp16
+ *                           in the kernel for few rows.  Relative difference (2-norm) of two such results on N(0,1)
+ *                           inputs: fp16 4e-4, bf16 2e-3 (0.7e-3 with the two-term P), e4m3 2e-2 to 3e-2.  An explicit
+ *                           CFK_TUNE_FMHA_SCHED keeps every call in kernel 0, whose results do not depend on the other
+ *                           heads;
  *                           1 pairs of CTAs (two SMs per 256 rows, tcgen05 cta_group::2; 16-bit inputs with head
  *                           dimension 128 only, other shapes run kernel 0); 2 a persistent grid whose CTAs take one
  *                           128-row tile at a time, with the scores double-buffered, both softmax warpgroups on the
@@ -194,7 +202,8 @@ const char* cfk_last_cuda_error(void);
  *   CFK_TUNE_FMHA_SCHED     kernel 0 at head dimension 128: how the two query tiles of a CTA use tensor memory.
  *                           0: each has a score buffer and writes its probabilities over it; 1: they take turns on
  *                           one score buffer and keep their probabilities in buffers of their own, so that no
- *                           Q K^T waits for a P V; -1 (default): by input type, the measured best.
+ *                           Q K^T waits for a P V; -1 (default): by input type, the measured best (1 for e4m3, else 0).
+ *                           0 or 1, at any head dimension, also keeps a call in kernel 0 whatever its size.
  */
 enum cfk_tunable { CFK_TUNE_FMHA_EXP_EMU = 0, CFK_TUNE_FMHA_GROUP_MB = 1, CFK_TUNE_FMHA_KERNEL = 2, CFK_TUNE_FMHA_GRID = 3,
                    CFK_TUNE_FMHA_SCHED = 4, CFK_TUNE_COUNT = 5 };

@@ -170,6 +170,46 @@ def test_fmha_shard_plan_union_is_bit_identical_to_the_unsharded_launch(lib, cud
     assert torch.equal(o, o_full) and torch.equal(lse, lse_full)
 
 
+# largest relative difference (2-norm) between two results of the stated accuracy, each within 3e-4 (fp16: P and O rounded to 11
+# bits), 1.7e-3 (bf16, P to 8 bits), 2.7e-2 (e4m3, P to 4 bits) of the exact one with independent errors: sqrt(2) times that, and 1.2
+CUT_DIFF = {0: 5.1e-4, 1: 2.9e-3, 2: 4.6e-2}
+
+
+@pytest.mark.parametrize("dtype,D", [(0, 64), (0, 128), (1, 128), (2, 64), (2, 128)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_fmha_shard_union_where_the_ranks_split_the_keys(lib, cuda, dtype, D, causal):
+    """32 heads in one call run with whole keys, 4 heads (a rank of 8) in four parts: the union of the ranks differs from the
+    unsharded launch by the rounding of P, and equals it bit for bit under an explicit schedule."""
+    import bench
+    from cfk_b200 import TUNE_FMHA_SCHED
+    from helpers import BLOCK, ONE_TILE, fmha_plan
+    B, S, H, world = 1, 2048, 32, 8
+    wl = (dtype, B, H, S, D, causal, "shard test")
+    low, _, scales = make_qkv(dtype, B, S, S, H, D, seed=17)
+    q, k, v = (x.cuda() for x in low)
+
+    def union(ranks):
+        o = torch.full((B, S, H, D), -1.0, dtype=torch.float16, device="cuda")
+        lse = torch.full((B, H, S), -1.0, dtype=torch.float32, device="cuda")
+        for rank in range(ranks):
+            bench.run_plan(lib, wl, bench.shard_plan(B, H, ranks, rank), q, k, v, o, scales, lse)
+        lib.check_device()
+        return o, lse
+
+    assert fmha_plan(lib, dtype, B, H, S, S, D, causal) == (BLOCK, 0, 0, 0)
+    assert fmha_plan(lib, dtype, B, H // world, S, S, D, causal) == (ONE_TILE, 4, 0, 0)
+    (one, lse_one), (cut, lse_cut) = union(1), union(world)
+    assert float((one.float() - cut.float()).norm() / one.float().norm()) < CUT_DIFF[dtype]
+    assert float((lse_one - lse_cut).abs().max()) < (2e-3 if dtype == 2 else 1e-4)
+    try:
+        lib.set_tunable(TUNE_FMHA_SCHED, 1 if dtype == 2 else 0)        # the defaults of the types
+        (one_b, lse_one_b), (cut_b, lse_cut_b) = union(1), union(world)
+    finally:
+        lib.set_tunable(TUNE_FMHA_SCHED, -1)
+    assert torch.equal(one, one_b) and torch.equal(one, cut_b)
+    assert torch.equal(lse_one, lse_one_b) and torch.equal(lse_one, lse_cut_b)
+
+
 def test_fmha_is_deterministic_and_iterations_repeat(lib, cuda):
     low, _, scales = make_qkv(0, 1, 1024, 1024, 2, 128, seed=2)
     a, _ = run_fmha(lib, low, scales, 0, True, want_stats=False)
