@@ -540,8 +540,7 @@ def main():
                    "sub_calls_per_step": len(plan)},
         "roofline": {"bound": "tensor", "achieved": per_gpu, "peak": burst, "unit": "TFLOP/s", "frac": per_gpu / burst,
                      "traffic": NCU_DRAM_BYTES_PER_LAUNCH.get(args.workload) if world == 1 else None,
-                     "traffic_source": "one ncu capture of the same shape, not of this run: "
-                                       "profiles/fmha_fwd_kernel_c3_c4_c5.md" if world == 1 else None,
+                     "traffic_source": "one ncu capture of the same shape, not of this run" if world == 1 else None,
                      "peak_source": f"{peak_kind} {'e4m3 UMMA' if dt == 2 else 'bf16 GEMM'} burst "
                                     f"(timed region {region_ms:.0f} ms)",
                      "umma_peak_live": {"what": "dense tcgen05.mma 128x256 from shared memory, all SMs, this run", **probes},

@@ -203,7 +203,7 @@ extern "C" int cfk_fill(void* dst, int dtype, int64_t n, uint64_t seed, int64_t 
   if (n == 0) return CFK_OK;
   const int threads = 256;
   const int64_t want = (n + threads - 1) / threads;
-  const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
+  const int blocks = (int)(want < kSMs * 16 ? want : kSMs * 16);
   return note_cuda(launch_overlapped(fill_kernel, blocks, threads, 0, (cudaStream_t)stream, dst, dtype, n, seed, first_index,
                                      kind, scale, value), "fill launch") == cudaSuccess ? CFK_OK : CFK_ERR_LAUNCH;
 }
@@ -237,7 +237,6 @@ static bool resolve_strides(const int64_t in[3], int64_t out[3], int S, int H, i
 //   54 / 66, 32 x 8192: 212 / 257; 222 and 297 heads 53 / 44 and 76 / 70.  Not so with the two-term P of bf16, which costs the
 //   256-row kernel more (256 heads, 32 x 800: 38 / 36), and with e4m3 V (256 heads, 32 x 4096: 84 / 79).
 static bool decode_is_faster(const cfk_fmha_args* a) {
-  constexpr int kSMs = 148;
   const int sq = a->seqlen_q, skv = a->seqlen_kv;
   const long long bh = (long long)a->batch * a->heads, groups = bh * ((sq + 15) / 16);
   if (groups > 0x7fffffffLL / 8) return false;
@@ -264,10 +263,10 @@ static int decode_splits(long long groups, int ntiles, int resident) {
 
 // One 128-row tile per CTA, two CTAs per SM (fmha_fwd_tile_sm100.cuh), against one 256-row block per SM
 // (fmha_fwd_sm100.cuh).  Returns the number of CTAs that share a tile's keys, 0 for the 256-row kernel.
-//   Fewer tiles than CTAs fit on the chip, and at least 8 key tiles: the keys are split as far as the chip has room, two key
-//   tiles per CTA at least, eight where there is room for two parts only (8 heads, 1024 x 1024 in two: 18.4 against 17.0).  us, bf16 d = 128 causal, 256-row kernel / whole keys / split: 8 heads, 256 x 2048 28.4 / 25.4 /
-//   13.7 (8 parts), 512 x 4096 51.2 / 46.3 / 18.8 (8), 2048 x 2048 29.0 / 28.2 / 25.9 (2); 24 heads, 512 x 4096 52.1 / 51.6 /
-//   40.9 (2).
+//   Fewer tiles than CTAs fit on the chip, and at least 8 key tiles (897 keys): the keys are split as far as the chip has room,
+//   two key tiles per CTA at least, eight where there is room for two parts only (8 heads, 1024 x 1024 in two: 18.4 against
+//   17.0).  us, bf16 d = 128 causal, 256-row kernel / whole keys / split: 8 heads, 256 x 2048 28.4 / 25.4 / 13.7 (8 parts),
+//   512 x 4096 51.2 / 46.3 / 18.8 (8), 2048 x 2048 29.0 / 28.2 / 25.9 (2); 24 heads, 512 x 4096 52.1 / 51.6 / 40.9 (2).
 //   Otherwise short keys, up to 12 tiles: the estimate below decides, with 6 % in favour of the 256-row kernel.  300 heads,
 //   128 x 128 18.0 / 12.3, 300 x 300 48.4 / 33.7; 100 heads, 640 x 640 34.2 / 24.4.  With longer keys the 256-row kernel, which
 //   reads K and V once per 256 rows, is as fast or faster: 8 heads, 8192 x 8192 107.5 / 120.0.
@@ -294,11 +293,10 @@ static float estimate_us(const cfk_fmha_args* a, int rows, int slots, const Tile
 // can cost a wave of its own.  It then runs in the few-rows kernel, as a second launch (about 4 us, and the cache once per 16
 // rows at 1.4 times the copy rate), where the estimate says that the wave it saves is worth clearly more.  us, one launch /
 // two: bf16 d = 128, 12 heads, 3080 x 3080: 83.4 / 55.6, 48 heads, 777 x 1300: 44.0 / 40.2, 75 heads, 258 x 1600: 46.7 / 39.1.
-// Below 1024 keys the second launch eats the gain (100 heads, 257 x 400: 25.3 / 26.2), and causal calls, whose CTAs differ in
+// With short keys the second launch eats the gain, so it is taken from 8 key tiles (897 keys) on (100 heads, 257 x 400: 25.3 / 26.2), and causal calls, whose CTAs differ in
 // length anyway, lost (48 heads, 777 x 1300: 43.0 / 46.1).
 struct TilePlan { int splits, tail_rows; };   // splits 0: the 256-row kernel
 static TilePlan tile_plan(const cfk_fmha_args* a) {
-  constexpr int kSMs = 148;
   const long long bh = (long long)a->batch * a->heads, units = bh * ((a->seqlen_q + 127) / 128);
   const int nall = (a->seqlen_kv + 127) / 128;
   if (nall >= 8 && 2 * units <= 2 * kSMs) {
@@ -358,7 +356,7 @@ struct FmhaChoice {
 static int few_rows_splits(const cfk_fmha_args* a, int rows) {
   const int esz = dtype_size(a->dtype), vsz = dtype_size(v_dtype(a)), keys = decode_tile_keys(a->head_dim, vsz);
   return decode_splits((long long)a->batch * a->heads * ((rows + 15) / 16), (a->seqlen_kv + keys - 1) / keys,
-                       148 * decode_ctas_per_sm(a->head_dim, esz, vsz));
+                       kSMs * decode_ctas_per_sm(a->head_dim, esz, vsz));
 }
 static FmhaChoice choose_kernel(const cfk_fmha_args* a) {
   tunables_from_env();

@@ -10,8 +10,9 @@
 //
 // A query tile of 16 rows is what mma.sync.m16n8k16 takes; a tcgen05.mma has at least 64 rows, and its way through tensor
 // memory costs more than the arithmetic, which needs a fraction of the time the bytes take.  One row against 6001 keys, 128
-// heads, d = 128, bf16 (393 MB): 62.9 us, 6.2 TB/s, against 70.6 in the 256-row kernel; d = 64: 35.1 against 57.7; e4m3:
-// 36.5 against 61.4; 2 heads x 65536 keys: 57.5 against 679 (the rule and more figures: capi.cu, decode_is_faster).  Every warp keeps a maximum, a sum
+// heads, d = 128, bf16 (393 MB): 61 us, 6.4 TB/s, against 70.6 in the 256-row kernel with the same launches; d = 64: 35.1
+// against 57.7; e4m3: 36.5 against 61.4; 2 heads x 65536 keys: 57.5 against 679 (the rule and more figures: capi.cu,
+// decode_is_faster).  Every warp keeps a maximum, a sum
 // and an output of its own, so nothing synchronises inside the loop; at the end the four are merged through shared memory and
 // the CTAs of one (batch, head), which form a cluster, through distributed shared memory.  So there is no workspace in global
 // memory, no second launch, and calls on several streams share nothing.
@@ -26,9 +27,9 @@ template <int DT, int PT, int HD>
 struct DecodeCfg {
   static constexpr int ESZ = (DT == kDtE4M3) ? 1 : 2, PESZ = (PT == kDtE4M3) ? 1 : 2;
   static constexpr int ROWS = 16, NWARP = 4;
-  // Keys per tile: a round of the producer (wait for the slot, announce the bytes, issue the copies) takes about 160 ns
-  // however small the tile is, so short rows travel 128 at a time (d = 64, 16 bit, one CTA: 322 us for 65536 keys with
-  // 64-key copies on barriers of their own).
+  // Keys per tile: a round of the producer (wait for the slot, announce the bytes, issue the copies) takes the same time however
+  // small the tile is, so short rows travel 128 at a time: d = 64, 16 bit, one CTA, 65536 keys as 2048 copies of 64 keys with a
+  // barrier each: 322 us, 0.16 per round.
   static constexpr int ROWB = HD * ESZ, SPANB = ROWB < 128 ? ROWB : 128;
   static constexpr int VROWB = HD * PESZ, VSPANB = VROWB < 128 ? VROWB : 128;
   static constexpr int TN = decode_tile_keys(HD, PESZ), NK = TN / NWARP, NT = NK / 8;   // keys and 8-key columns per warp

@@ -23,7 +23,7 @@ int decode_launch(const FmhaLaunch& L) {
   dp.p = L.p;
   const int ntiles = (L.p.Skv + C::TN - 1) / C::TN;
   const long long ctas = (long long)dp.splits * dp.nqb * L.p.H * L.p.B;
-  dp.nslot = C::slots(ctas, 148, (ntiles + dp.splits - 1) / dp.splits);
+  dp.nslot = C::slots(ctas, kSMs, (ntiles + dp.splits - 1) / dp.splits);
   const dim3 grid((unsigned)ctas, 1, 1);
   for (int it = 0; it < L.iterations; ++it)
     if (note_cuda(launch_overlapped_in(dp.splits, kern, grid, dim3(C::NTHREADS), C::smem_bytes(dp.nslot, L.p.Sq), L.stream, L.tm_q, L.tm_k,

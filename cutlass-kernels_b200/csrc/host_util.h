@@ -44,6 +44,9 @@ inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 blo
   return launch_overlapped_in(1, kern, grid, block, smem, stream, args...);
 }
 
+// SMs of the one device this library is built for.  Only the choice between kernels and the sizes of grids follow from it.
+constexpr int kSMs = 148;
+
 // Device pointer to the 256-byte status block of the current device (int[64]; word 0 is the status
 // word the kernels write).  nullptr (and *err set) if there is no usable device.
 int* device_status_block(int* err);
