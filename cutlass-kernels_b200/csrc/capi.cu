@@ -267,9 +267,9 @@ static int decode_splits(long long groups, int ntiles, int resident) {
 //   two key tiles per CTA at least, eight where there is room for two parts only (8 heads, 1024 x 1024 in two: 18.4 against
 //   17.0).  us, bf16 d = 128 causal, 256-row kernel / whole keys / split: 8 heads, 256 x 2048 28.4 / 25.4 / 13.7 (8 parts),
 //   512 x 4096 51.2 / 46.3 / 18.8 (8), 2048 x 2048 29.0 / 28.2 / 25.9 (2); 24 heads, 512 x 4096 52.1 / 51.6 / 40.9 (2).
-//   Otherwise short keys, up to 12 tiles: the estimate below decides, with 6 % in favour of the 256-row kernel.  300 heads,
-//   128 x 128 18.0 / 12.3, 300 x 300 48.4 / 33.7; 100 heads, 640 x 640 34.2 / 24.4.  With longer keys the 256-row kernel, which
-//   reads K and V once per 256 rows, is as fast or faster: 8 heads, 8192 x 8192 107.5 / 120.0.
+//   Otherwise short keys, up to 12 tiles: the estimate below decides, with 6 % in favour of the 256-row kernel.  Causal,
+//   300 heads, 128 x 128 18.0 / 12.3, 300 x 300 48.4 / 33.7; 100 heads, 640 x 640 34.2 / 24.4.  With longer keys the 256-row
+//   kernel, which reads K and V once per 256 rows, is as fast or faster: 8 heads, 8192 x 8192 107.5 / 120.0.
 // The estimate, in us: a fixed time per CTA, a time per key tile, and for causal calls the tail of the heaviest-first order;
 // the constants are fits to a sweep of 24 shapes x causal or not for each type (root mean square error 6-13 %).
 struct TileCost { float fixed, per_tile, tail, offset; };

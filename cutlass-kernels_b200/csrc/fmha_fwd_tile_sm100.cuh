@@ -8,7 +8,7 @@
 //
 // A CTA takes half an SM: 256 columns of tensor memory, at most 113 KB of shared memory, half the registers.  Two CTAs on an
 // SM interleave as the two query tiles of the 256-row kernel do, but start and end on their own: the work comes in half the
-// pieces, and the last wave in halves of SMs: 300 heads of 300 x 300, bf16 d = 128: 48.4 -> 33.7 us.  K and V are read once
+// pieces, and the last wave in halves of SMs: 300 heads of 300 x 300, bf16 d = 128 causal: 48.4 -> 33.7 us.  K and V are read once
 // per 128 rows instead of per 256, which is why long calls stay with the 256-row kernel.
 //
 // Where even the 128-row tiles are too few, a cluster of `splits` CTAs shares one: each takes a contiguous part of the key
