@@ -71,3 +71,40 @@ def test_narrow_and_split_plans_in_tf32_with_a_separate_source(lib, cuda, M, N, 
     err = np.abs(d[:L * M * N].view(*shape).cpu().numpy() - ref).max()
     assert err <= K * 2.0 ** -24 * K ** 0.5 / 2 + 2.0 ** -22, err
     assert bool((d[L * M * N:] == -3.0).all())
+
+
+def test_threads_on_streams_of_their_own_get_the_plans_and_results_of_one(lib, cuda):
+    import threading
+    g = torch.Generator().manual_seed(2)
+    calls = []
+    for i, (M, N, K, L, row_major) in enumerate(SHAPES[:12]):
+        a, b = (torch.randn(L, r, K, generator=g).bfloat16().cuda() for r in (M, N))
+        c, d = (torch.zeros(L, M, N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        calls.append((a, b, c, d, dict(dtype=1, m=M, n=N, k=K, l=L, c_row_major=row_major)))
+    torch.cuda.synchronize()
+    plans, errors = {}, []
+
+    def work(i):
+        try:
+            torch.cuda.set_device(0)
+            a, b, c, _, kw = calls[i]
+            plans[i] = gemm_plan(lib, *SHAPES[i], dtype=1)
+            stream = torch.cuda.Stream()
+            for _ in range(3):
+                lib.gemm(a, b, c, **kw, stream=stream.cuda_stream)
+            stream.synchronize()
+        except Exception as e:      # noqa: BLE001 - reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    lib.check_device()
+    assert [plans[i] for i in range(len(calls))] == PLANS[:len(calls)]
+    for a, b, c, d, kw in calls:
+        lib.gemm(a, b, d, **kw)
+        lib.check_device()
+        assert torch.equal(c, d)
